@@ -46,6 +46,10 @@ struct Geometry {
   // the bulk entry's constants, so the step kernel takes them from the kernel
   // argument instead of loading them from the cell's table entry
   int32_t uniform;
+  // flat tiles of the step kernels: 0 or the multiplier and shift of
+  // floor(n / nz) = (mulhi(n, flat_mul) + n) >> flat_shift (tile_cells)
+  int32_t flat;
+  uint32_t flat_mul, flat_shift;
 };
 
 // the entry index the masked kernels give a cell of the bulk box (the table
@@ -225,6 +229,16 @@ constexpr StepVariant kStepVariants[] = {{1, 3}, {1, 4}, {2, 2}, {2, 3}};
 #endif
 constexpr int kNumStepVariants = 4;
 
+// Variant v for a storage element of `bytes`.  16-bit storage compiles the
+// one-cell-per-thread variants only (its kernels hold two cells per thread
+// already; at 256^3 two elements per thread reached 0.87 of the copy bandwidth
+// against 0.94 with one in D3Q19, 0.87 against 0.93 in D3Q27), so the ids of
+// the others give the one-cell variant of the same rank.
+constexpr StepVariant step_variant(int bytes, int v)
+{
+  return kStepVariants[bytes == 2 ? v & 1 : v];
+}
+
 // running sums of the fused statistics of one thread
 struct StatAcc {
   double rho = 0., usqr = 0., max = 0.;
@@ -239,12 +253,47 @@ struct StatAcc {
   }
 };
 
-// One tile of the step: the CPT cells (x, y0 + k*dy, z) of this thread.
-// Masked lattices pass each cell's table entry in id[k] (loaded a tile ahead by
-// aa_step_masked_kernel); unmasked lattices use `bulk` for every cell.
+// The (y, z) of this thread's CPT cells.  Two ways to cut a plane x into blocks:
+//   rectangles  blockDim.x cells along z by blockDim.y * CPT rows (the launch
+//               shape); lanes beyond nz and rows beyond ny idle;
+//   flat        CPT runs of kStepThreads consecutive cells of the plane's
+//               index y*nz + z, so every lane but the plane's last few has a
+//               cell, whatever nz and ny; y costs one multiply-high
+//               (Granlund & Montgomery, PLDI 1994).
+// Lanes without a cell get y = ny.
+OLB_DEV void flat_cell(const Geometry& g, uint32_t n, int& y, int& z)
+{
+  const uint32_t yy = (__umulhi(n, g.flat_mul) + n) >> g.flat_shift;
+  z = int(n - yy * uint32_t(g.nz));
+  y = n < uint32_t(g.ny) * uint32_t(g.nz) ? int(yy) : g.ny;
+}
+
+template <int CPT>
+OLB_DEV void tile_cells(const Geometry& g, int (&y)[CPT], int (&z)[CPT])
+{
+  if (g.flat) {
+    static_for<0, CPT>([&](auto k) {
+      const uint32_t n = (blockIdx.x * uint32_t(CPT) + uint32_t(k.value)) * uint32_t(kStepThreads) + threadIdx.x;
+      flat_cell(g, n, y[k], z[k]);
+    });
+  } else {
+    const int zz = blockIdx.x * blockDim.x + threadIdx.x;
+    static_for<0, CPT>([&](auto k) {
+      z[k] = zz;
+      y[k] = zz < g.nz ? int(blockIdx.y * (blockDim.y * CPT) + threadIdx.y + k.value * blockDim.y) : g.ny;
+      y[k] = min(y[k], g.ny);
+    });
+  }
+}
+
+// One tile of the step: the CPT cells (x, y[k], z[k]) of this thread (none
+// where y[k] = ny).  Masked lattices pass each cell's table entry in id[k]
+// (loaded ahead by aa_step_masked_kernel); unmasked lattices use `bulk` for
+// every cell.
 template <int Q, class S, class R, int KIND, bool ODD, bool MASKED, bool STATS, int CPT>
 OLB_DEV void step_tile(S* __restrict__ pops, const Geometry& g, const DynDevice<R>* __restrict__ table,
-                       const DynDevice<R>& bulk, int x, int y0, int z, int dy, const int (&id)[CPT], StatAcc& acc)
+                       const DynDevice<R>& bulk, int x, const int (&y)[CPT], const int (&z)[CPT],
+                       const int (&id)[CPT], StatAcc& acc)
 {
   using L = Lattice<Q>;
   using ST = Store<S, R>;
@@ -260,13 +309,12 @@ OLB_DEV void step_tile(S* __restrict__ pops, const Geometry& g, const DynDevice<
   // together instead of one after the other); a full-way bounce-back cell
   // then stores nothing, its AA update being a no-op (see file comment).
   static_for<0, CPT>([&](auto k) {
-    const int y = y0 + k.value * dy;
-    go[k] = z < g.nz && y < g.ny;
+    go[k] = y[k] < g.ny;
     kind[k] = KIND;
     n[k] = 0;
     if (go[k]) {
-      n[k] = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y)) * uint32_t(g.nz) + uint32_t(z);
-      Neighbours nb(g, x, y, z);
+      n[k] = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k]);
+      Neighbours nb(g, x, y[k], z[k]);
       static_for<0, Q>([&](auto i) {
         if constexpr (!ODD) {
           f[k][i] = ST::template load<L, i.value>(pops + size_t(i.value) * g.stride + n[k]);
@@ -297,7 +345,6 @@ OLB_DEV void step_tile(S* __restrict__ pops, const Geometry& g, const DynDevice<
   // phase 2: collide and store
   static_for<0, CPT>([&](auto k) {
     if (!go[k]) return;
-    const int y = y0 + k.value * dy;
     R st_rho = R(0), st_usqr = R(0);
     bool counted = false;
     if (kind[k] == KIND) {
@@ -361,7 +408,7 @@ OLB_DEV void step_tile(S* __restrict__ pops, const Geometry& g, const DynDevice<
     // pass through unchanged.
     // The store offsets are recomputed here rather than kept live through
     // the collision.
-    Neighbours nb(g, int(opaque(uint32_t(x))), int(opaque(uint32_t(y))), int(opaque(uint32_t(z))));
+    Neighbours nb(g, int(opaque(uint32_t(x))), int(opaque(uint32_t(y[k]))), int(opaque(uint32_t(z[k]))));
     const uint32_t stride = opaque(g.stride);
     const uint32_t nk = opaque(n[k]);
     static_for<0, Q>([&](auto i) {
@@ -385,12 +432,11 @@ template <int Q, class S, class R, int KIND, bool ODD, bool STATS, int CPT, int 
 __global__ void __launch_bounds__(kStepThreads, MINB)
 aa_step_kernel(S* __restrict__ pops, const Geometry g, const DynDevice<R> bulk, StatPartial* __restrict__ partials)
 {
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y0 = blockIdx.y * (blockDim.y * CPT) + threadIdx.y;
-  const int x = blockIdx.z;
+  int y[CPT], z[CPT];
+  tile_cells(g, y, z);
   const int none[CPT] = {};
   StatAcc acc;
-  step_tile<Q, S, R, KIND, ODD, false, STATS, CPT>(pops, g, nullptr, bulk, x, y0, z, int(blockDim.y), none, acc);
+  step_tile<Q, S, R, KIND, ODD, false, STATS, CPT>(pops, g, nullptr, bulk, int(blockIdx.z), y, z, none, acc);
   if constexpr (STATS) {
     block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
   }
@@ -399,16 +445,15 @@ aa_step_kernel(S* __restrict__ pops, const Geometry g, const DynDevice<R> bulk, 
 // table entries of a tile's cells: kBoxCell for cells of the bulk box (they
 // use the bulk entry, no load), -1 for cells outside the lattice (skipped)
 template <int CPT>
-OLB_DEV void load_tile_ids(int (&id)[CPT], const Geometry& g, const uint8_t* __restrict__ ids, int x, int y0,
-                           int z, int dy)
+OLB_DEV void load_tile_ids(int (&id)[CPT], const Geometry& g, const uint8_t* __restrict__ ids, int x,
+                           const int (&y)[CPT], const int (&z)[CPT])
 {
   static_for<0, CPT>([&](auto k) {
-    const int y = y0 + k.value * dy;
     id[k] = -1;
-    if (z < g.nz && y < g.ny) {
-      id[k] = in_bulk_box(g, x, y, z)
+    if (y[k] < g.ny) {
+      id[k] = in_bulk_box(g, x, y[k], z[k])
                 ? kBoxCell
-                : int(ids[(uint32_t(x) * uint32_t(g.ny) + uint32_t(y)) * uint32_t(g.nz) + uint32_t(z)]);
+                : int(ids[(uint32_t(x) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k])]);
     }
   });
 }
@@ -422,14 +467,12 @@ aa_step_masked_kernel(S* __restrict__ pops, const Geometry g, const uint8_t* __r
                       const DynDevice<R>* __restrict__ table, const DynDevice<R> bulk,
                       StatPartial* __restrict__ partials)
 {
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y0 = blockIdx.y * (blockDim.y * CPT) + threadIdx.y;
   const int x = blockIdx.z;
-  const int dy = int(blockDim.y);
-  int id[CPT];
-  load_tile_ids(id, g, ids, x, y0, z, dy);
+  int y[CPT], z[CPT], id[CPT];
+  tile_cells(g, y, z);
+  load_tile_ids(id, g, ids, x, y, z);
   StatAcc acc;
-  step_tile<Q, S, R, KIND, ODD, true, STATS, CPT>(pops, g, table, bulk, x, y0, z, dy, id, acc);
+  step_tile<Q, S, R, KIND, ODD, true, STATS, CPT>(pops, g, table, bulk, x, y, z, id, acc);
   if constexpr (STATS) {
     block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
   }
@@ -626,13 +669,13 @@ OLB_DEV bool collide_any(float (&f)[L::q], int kind, const DynDevice<float>* e, 
   return false;  // NoDynamics / bounce-back / boundary cells (collided ahead): no statistic here
 }
 
-// One tile of the paired step: the CPT element rows (x', y0 + k*dy, z) of
-// this thread, each the two cells x' and x' + nx/2.  Masked lattices pass the
+// One tile of the paired step: the CPT elements (x', y[k], z[k]) of this
+// thread (none where y[k] = ny), each the two cells x' and x' + nx/2.  Masked lattices pass the
 // table entries of both cells (loaded a tile ahead); unmasked ones use `bulk`.
 template <int Q, class S, int KIND, bool ODD, bool MASKED, bool STATS, int CPT>
 OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const DynDevice<float>* __restrict__ table,
-                         const DynDevice<float>& bulk, int xp, int y0, int z, int dy, const int (&id_lo)[CPT],
-                         const int (&id_hi)[CPT], StatAcc& acc)
+                         const DynDevice<float>& bulk, int xp, const int (&y)[CPT], const int (&z)[CPT],
+                         const int (&id_lo)[CPT], const int (&id_hi)[CPT], StatAcc& acc)
 {
   using L = Lattice<Q>;
   using P = Pair<S>;
@@ -649,15 +692,14 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
   uint32_t e[CPT];
 
   static_for<0, CPT>([&](auto k) {
-    const int y = y0 + k.value * dy;
-    go[k] = z < g.nz && y < g.ny;
+    go[k] = y[k] < g.ny;
     kind_lo[k] = kind_hi[k] = KIND;
     e[k] = 0;
     if (go[k]) {
       // the pair's populations are loaded before its ids have arrived (as in
       // step_tile); a pair of two bounce-back cells then stores nothing
-      e[k] = (uint32_t(xp) * uint32_t(g.ny) + uint32_t(y)) * uint32_t(g.nz) + uint32_t(z);
-      PairNeighbours nb(g, xp, y, z);
+      e[k] = (uint32_t(xp) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k]);
+      PairNeighbours nb(g, xp, y[k], z[k]);
       static_for<0, Q>([&](auto i) {
         // 32-bit element indices: the paired layout is only used while
         // q * pstride < 2^32 (olb_b200_create)
@@ -688,7 +730,6 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
 
   static_for<0, CPT>([&](auto k) {
     if (!go[k]) return;
-    const int y = y0 + k.value * dy;
     // the table entries (nullptr: the bulk entry, the kernel argument)
     const DynDevice<float>* pe_lo = MASKED && id_lo[k] != kBoxCell ? table + id_lo[k] : nullptr;
     const DynDevice<float>* pe_hi = MASKED && id_hi[k] != kBoxCell ? table + id_hi[k] : nullptr;
@@ -697,7 +738,7 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
     // dynamics; loaded here, after the populations)
     auto load_force = [&](int x, float (&fc)[3]) {
       const float* __restrict__ F = static_cast<const float*>(g.force);
-      const uint32_t nn = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y)) * uint32_t(g.nz) + uint32_t(z);
+      const uint32_t nn = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k]);
       fc[0] = __ldg(F + nn);
       fc[1] = __ldg(F + size_t(g.stride) + nn);
       fc[2] = __ldg(F + 2 * size_t(g.stride) + nn);
@@ -810,7 +851,7 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
     cell(std::integral_constant<bool, true>{}, kind_hi[k], pe_hi);
     }
     // recomputed after the collision rather than kept live through it
-    PairNeighbours nb(g, int(opaque(uint32_t(xp))), int(opaque(uint32_t(y))), int(opaque(uint32_t(z))));
+    PairNeighbours nb(g, int(opaque(uint32_t(xp))), int(opaque(uint32_t(y[k]))), int(opaque(uint32_t(z[k]))));
     const uint32_t ps = opaque(pstride);
     const uint32_t ek = opaque(e[k]);
     static_for<0, Q>([&](auto i) {
@@ -834,13 +875,11 @@ __global__ void __launch_bounds__(kStepThreads, MINB)
 aa_step_paired_kernel(S* __restrict__ pops, const Geometry g, const DynDevice<float> bulk,
                       StatPartial* __restrict__ partials)
 {
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y0 = blockIdx.y * (blockDim.y * CPT) + threadIdx.y;
-  const int xp = blockIdx.z;
+  int y[CPT], z[CPT];
+  tile_cells(g, y, z);
   const int none[CPT] = {};
   StatAcc acc;
-  paired_tile<Q, S, KIND, ODD, false, STATS, CPT>(pops, g, nullptr, bulk, xp, y0, z, int(blockDim.y), none, none,
-                                                 acc);
+  paired_tile<Q, S, KIND, ODD, false, STATS, CPT>(pops, g, nullptr, bulk, int(blockIdx.z), y, z, none, none, acc);
   if constexpr (STATS) {
     block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
   }
@@ -853,15 +892,13 @@ aa_step_masked_paired_kernel(S* __restrict__ pops, const Geometry g, const uint8
                              const DynDevice<float>* __restrict__ table, const DynDevice<float> bulk,
                              StatPartial* __restrict__ partials)
 {
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y0 = blockIdx.y * (blockDim.y * CPT) + threadIdx.y;
   const int xp = blockIdx.z;
-  const int dy = int(blockDim.y);
-  int lo[CPT], hi[CPT];
-  load_tile_ids(lo, g, ids, xp, y0, z, dy);
-  load_tile_ids(hi, g, ids, xp + (g.nx >> 1), y0, z, dy);
+  int y[CPT], z[CPT], lo[CPT], hi[CPT];
+  tile_cells(g, y, z);
+  load_tile_ids(lo, g, ids, xp, y, z);
+  load_tile_ids(hi, g, ids, xp + (g.nx >> 1), y, z);
   StatAcc acc;
-  paired_tile<Q, S, KIND, ODD, true, STATS, CPT>(pops, g, table, bulk, xp, y0, z, dy, lo, hi, acc);
+  paired_tile<Q, S, KIND, ODD, true, STATS, CPT>(pops, g, table, bulk, xp, y, z, lo, hi, acc);
   if constexpr (STATS) {
     block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
   }
@@ -1432,10 +1469,47 @@ cudaError_t launch_boundary(void* pops, const Geometry& g, bool shifted, const u
                             int periodic, const uint32_t* cells, uint32_t n_flat, uint32_t n_edge,
                             uint32_t n_corner, cudaStream_t stream);
 
+// grid of the step kernels: flat tiles, or rectangles of bz x (by * cells per thread)
 inline dim3 step_grid(const Geometry& g, int bz, int by, int cells_per_thread)
 {
+  const unsigned planes = unsigned(g.paired ? g.nx / 2 : g.nx);
+  if (g.flat) {
+    const uint64_t tile = uint64_t(kStepThreads) * uint64_t(cells_per_thread);
+    return dim3(unsigned((uint64_t(g.ny) * uint64_t(g.nz) + tile - 1) / tile), 1, planes);
+  }
   const int rows = by * cells_per_thread;
-  return dim3((g.nz + bz - 1) / bz, (g.ny + rows - 1) / rows, g.paired ? g.nx / 2 : g.nx);
+  return dim3((g.nz + bz - 1) / bz, (g.ny + rows - 1) / rows, planes);
+}
+
+// Whether an unfixed launch shape gives way to flat tiles.  Rectangles leave
+// lanes without cells when nz or ny is no multiple of theirs: 0.58 of the lanes
+// have cells at 191x173x150, and flat tiles take 125 us against 144 (cavity,
+// FP32), 31 against 35 at 200x120x100 (FP16, 0.78 of the lanes), 12.3 against
+// 15.4 at 97x61x75.  With every lane busy (256^3) FP32 and FP64 still gain
+// 0.1 % to 3 % (389 us against 402: a block's loads are one contiguous run of
+// every column), 16-bit storage loses 1 % to 3 % (D3Q27 BF16 312 us against
+// 302: the division by nz on an issue-bound kernel) and keeps rectangles.
+inline bool use_flat_tiles(const Geometry& g, int bytes, int bz, int by, int cells_per_thread)
+{
+  if (bytes > 2) return true;
+  const uint64_t rows = uint64_t(by) * uint64_t(cells_per_thread);
+  const uint64_t lanes = (uint64_t(g.nz) + bz - 1) / bz * bz * ((uint64_t(g.ny) + rows - 1) / rows * rows);
+  return 100 * uint64_t(g.ny) * uint64_t(g.nz) < 97 * lanes;
+}
+
+inline dim3 step_block(const Geometry& g, int bz, int by)
+{
+  return g.flat ? dim3(kStepThreads, 1) : dim3(bz, by);
+}
+
+// the constants of the flat tiles' division by nz
+inline void set_flat(Geometry& g)
+{
+  uint32_t s = 0;
+  while ((uint64_t(1) << s) < uint64_t(g.nz)) ++s;
+  g.flat = 1;
+  g.flat_mul = uint32_t(((uint64_t(1) << 32) * ((uint64_t(1) << s) - uint64_t(g.nz))) / uint64_t(g.nz) + 1);
+  g.flat_shift = s;
 }
 
 // grid of the gather / moments kernels (one cell per thread)

@@ -13,7 +13,7 @@ namespace olb_b200 {
 template <int Q, class S, class R, int KIND, int CPT, int MINB>
 static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool masked, bool stats)
 {
-  const dim3 block(a.block_z, a.block_y);
+  const dim3 block = step_block(a.g, a.block_z, a.block_y);
   const dim3 grid = step_grid(a.g, a.block_z, a.block_y, CPT);
   S* pops = static_cast<S*>(a.pops);
   const DynDevice<R>* table = static_cast<const DynDevice<R>*>(a.table);
@@ -64,8 +64,8 @@ template <int Q, class S, class R, int KIND>
 static cudaError_t launch_step_kind(const StepLaunch& a, bool odd, bool masked, bool stats)
 {
 #define OLB_VARIANT(V)                                                                             \
-  launch_step_variant<Q, S, R, KIND, kStepVariants[V].cells_per_thread, kStepVariants[V].min_blocks>( \
-    a, odd, masked, stats)
+  launch_step_variant<Q, S, R, KIND, step_variant(sizeof(S), V).cells_per_thread,                  \
+                      step_variant(sizeof(S), V).min_blocks>(a, odd, masked, stats)
   switch (a.variant) {
   case 0: return OLB_VARIANT(0);
   case 1: return OLB_VARIANT(1);

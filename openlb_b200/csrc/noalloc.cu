@@ -130,19 +130,28 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   if (cells > (size_t(1) << 31)) return noalloc_fail(OLB_B200_ERR_ARG, "collide_and_stream_noalloc: too many cells");
 
   Geometry g{desc->nx, desc->ny, desc->nz, uint32_t((cells + 63) / 64 * 64)};
+  const bool f64 = desc->storage == OLB_B200_STORAGE_F64;
+  const int elem = f64 ? 8 : (desc->storage == OLB_B200_STORAGE_F32 ? 4 : 2);
   // the library's default launch shape
   const int bz = desc->nz >= 128 ? 128 : (desc->nz >= 64 ? 64 : 32);
   const int by = 256 / bz;
   // one cell per thread (step variant 0): 65536 blocks cover 256^3 cells
   const int variant = 0;
-  const dim3 grid = step_grid(g, bz, by, kStepVariants[variant].cells_per_thread);
-  const size_t blocks = size_t(grid.x) * grid.y * grid.z;
+  const int cells_per_thread = step_variant(elem, variant).cells_per_thread;
+  const dim3 rect = step_grid(g, bz, by, cells_per_thread);
+  size_t blocks = size_t(rect.x) * rect.y * rect.z;
   if (stats && blocks > kMaxBlocks) {
     char buf[256];
     snprintf(buf, sizeof buf, "collide_and_stream_noalloc: with statistics the lattice needs "
              "ceil(nz/%d)*ceil(ny/%d)*nx = %zu reduction blocks; the fixed scratch holds %zu",
              bz, by, blocks, kMaxBlocks);
     return noalloc_fail(OLB_B200_ERR_ARG, buf);
+  }
+  // the limit above is the documented one; flat tiles need no more blocks
+  if (use_flat_tiles(g, elem, bz, by, cells_per_thread)) {
+    set_flat(g);
+    const dim3 grid = step_grid(g, bz, by, cells_per_thread);
+    blocks = size_t(grid.x) * grid.y * grid.z;
   }
 
   cudaError_t e = cudaSetDevice(desc->device);
@@ -151,7 +160,6 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   olb_b200_status st = scratch_address(desc->device, &scratch);
   if (st != OLB_B200_OK) return st;
 
-  const bool f64 = desc->storage == OLB_B200_STORAGE_F64;
   alignas(16) unsigned char params[sizeof(DynDevice<double>)];
   if (f64) {
     const DynDevice<double> d = detail::device_params_f64(desc->q, *bulk);

@@ -265,7 +265,9 @@ struct olb_b200_lattice {
   StatPartial* stat_dev = nullptr;
   StatPartial* stat_host = nullptr;  // pinned
   int block_z = 0, block_y = 0;
-  int variant = 0;          // index into kStepVariants
+  int variant = 0;          // index of the step-kernel variant (step_variant)
+  bool shape_fixed = false; // block_z, block_y (or flat tiles) chosen by the caller or the autotuner
+  bool flat_fixed = false;  // the autotuner chose flat tiles
   void* force = nullptr;    // FORCE per cell, 3 columns of `stride` R (olb_b200_set_force_field)
   bool tuned = false;       // variant and shape chosen by olb_b200_autotune
   float tuned_ms = 0.f;
@@ -327,7 +329,19 @@ int default_variant(const olb_b200_lattice* L)
   return 3;                                                                          // {2,3}
 }
 
-int cells_per_thread(const olb_b200_lattice* L) { return kStepVariants[L->variant].cells_per_thread; }
+int cells_per_thread(const olb_b200_lattice* L)
+{
+  return step_variant(int(L->elem), L->variant).cells_per_thread;
+}
+
+// How the step kernels cut a plane: as fixed, else by use_flat_tiles.
+void choose_tiles(olb_b200_lattice* L)
+{
+  L->g.flat = 0;
+  const bool flat = L->shape_fixed ? L->flat_fixed
+                                   : use_flat_tiles(L->g, int(L->elem), L->block_z, L->block_y, cells_per_thread(L));
+  if (flat) set_flat(L->g);
+}
 
 template <class F>
 cudaError_t dispatch(const olb_b200_lattice* L, F&& f)
@@ -917,6 +931,7 @@ olb_b200_status olb_b200_set_dynamics(olb_b200_lattice* L, const uint8_t* ids,
     L->variant = default_variant(L);
     L->tuned = false;
   }
+  choose_tiles(L);
   return OLB_B200_OK;
 }
 
@@ -1140,6 +1155,8 @@ olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* L, int32_t block_z, 
   if (!L) return fail(OLB_B200_ERR_ARG, "set_launch_shape: null lattice");
   if (block_z == 0 && block_y == 0) {
     default_shape(L, L->block_z, L->block_y);
+    L->shape_fixed = L->flat_fixed = false;
+    choose_tiles(L);
     return OLB_B200_OK;
   }
   if (block_z < 32 || block_z % 32 != 0 || block_y < 1 || block_z * block_y > kStepThreads)
@@ -1147,6 +1164,9 @@ olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* L, int32_t block_z, 
                 "of 32, block_z*block_y <= %d", block_z, block_y, kStepThreads);
   L->block_z = block_z;
   L->block_y = block_y;
+  L->shape_fixed = true;
+  L->flat_fixed = false;
+  choose_tiles(L);
   return OLB_B200_OK;
 }
 
@@ -1292,6 +1312,7 @@ olb_b200_status olb_b200_set_step_variant(olb_b200_lattice* L, int32_t variant)
     return fail(OLB_B200_ERR_ARG, "set_step_variant: variant %d outside [-1, %d)", variant, kNumStepVariants);
   L->variant = variant < 0 ? default_variant(L) : variant;
   L->tuned = false;
+  choose_tiles(L);
   return OLB_B200_OK;
 }
 
@@ -1299,8 +1320,8 @@ olb_b200_status olb_b200_get_tuning(olb_b200_lattice* L, olb_b200_tuning* out)
 {
   if (!L || !out) return fail(OLB_B200_ERR_ARG, "get_tuning: null argument");
   out->variant = L->variant;
-  out->cells_per_thread = kStepVariants[L->variant].cells_per_thread;
-  out->min_blocks_per_sm = kStepVariants[L->variant].min_blocks;
+  out->cells_per_thread = step_variant(int(L->elem), L->variant).cells_per_thread;
+  out->min_blocks_per_sm = step_variant(int(L->elem), L->variant).min_blocks;
   out->block_z = L->block_z;
   out->block_y = L->block_y;
   out->tuned = L->tuned ? 1 : 0;
@@ -1332,18 +1353,27 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
   const int zmax = std::max(32, (L->desc.nz + 31) / 32 * 32);
   float best = 0.f;
   int best_v = L->variant, best_bz = L->block_z, best_by = L->block_y, tried = 0;
+  bool best_flat = L->g.flat != 0;
   for (int v = 0; v < kNumStepVariants && st == OLB_B200_OK; ++v) {
     bool duplicate = false;
     for (int w = 0; w < v; ++w) {
-      duplicate |= kStepVariants[w].cells_per_thread == kStepVariants[v].cells_per_thread &&
-                   kStepVariants[w].min_blocks == kStepVariants[v].min_blocks;
+      const StepVariant a = step_variant(int(L->elem), v), b = step_variant(int(L->elem), w);
+      duplicate |= a.cells_per_thread == b.cells_per_thread && a.min_blocks == b.min_blocks;
     }
     if (duplicate) continue;
-    for (int bz = 256; bz >= 32 && st == OLB_B200_OK; bz /= 2) {
+    // the rectangles of 256 threads, then (bz = 16) flat tiles
+    for (int bz = 256; bz >= 16 && st == OLB_B200_OK; bz /= 2) {
+      const bool flat = bz == 16;
       if (bz > zmax) continue;
       L->variant = v;
-      L->block_z = bz;
-      L->block_y = kStepThreads / bz;
+      if (flat) {
+        default_shape(L, L->block_z, L->block_y);
+        set_flat(L->g);
+      } else {
+        L->block_z = bz;
+        L->block_y = kStepThreads / bz;
+        L->g.flat = 0;
+      }
       st = enqueue_steps(L, 2, false);  // warm-up
       if (st != OLB_B200_OK) break;
       if ((e = cudaEventRecord(L->ev0, L->stream)) != cudaSuccess) { st = cuda_fail(e, "autotune event"); break; }
@@ -1361,8 +1391,9 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
       if (tried == 1 || ms < best) {
         best = ms;
         best_v = v;
-        best_bz = bz;
-        best_by = kStepThreads / bz;
+        best_bz = L->block_z;
+        best_by = L->block_y;
+        best_flat = flat;
       }
     }
   }
@@ -1372,12 +1403,16 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
   cudaFree(backup);
   L->parity = parity;
   L->steps_done = steps_done;
+  choose_tiles(L);
   if (st != OLB_B200_OK) return st;
   if (e != cudaSuccess) return cuda_fail(e, "autotune restore copy");
   if (e2 != cudaSuccess) return cuda_fail(e2, "autotune synchronize");
   L->variant = best_v;
   L->block_z = best_bz;
   L->block_y = best_by;
+  L->shape_fixed = true;
+  L->flat_fixed = best_flat;
+  choose_tiles(L);
   L->tuned = true;
   L->tuned_ms = best;
   if (out) {
