@@ -229,6 +229,16 @@ constexpr StepVariant kStepVariants[] = {{1, 3}, {1, 4}, {2, 2}, {2, 3}};
 #endif
 constexpr int kNumStepVariants = 4;
 
+// 16-bit storage in the natural layout (one cell per element) takes two cells
+// per thread as the lanes of the packed collision (aa_step_split_kernel); the
+// reference-order build collides one cell at a time
+#ifdef OLB_B200_EXACT
+constexpr bool kSplitNatural16 = false;
+#else
+constexpr bool kSplitNatural16 = true;
+#endif
+constexpr int kSplitMinBlocks = 3;
+
 // Variant v for a storage element of `bytes`.  16-bit storage compiles the
 // one-cell-per-thread variants only (its kernels hold two cells per thread
 // already; at 256^3 two elements per thread reached 0.87 of the copy bandwidth
@@ -669,6 +679,139 @@ OLB_DEV bool collide_any(float (&f)[L::q], int kind, const DynDevice<float>* e, 
   return false;  // NoDynamics / bounce-back / boundary cells (collided ahead): no statistic here
 }
 
+// Collision of two cells held as packed 16-bit pairs (low half: cell n_lo of
+// the natural order, high half: cell n_hi), in place; kind and table entry per
+// cell.  count_hi: the high cell enters the statistics.
+template <int Q, class S, int KIND, bool MASKED, bool STATS>
+OLB_DEV void collide_packed(typename Pair<S>::T (&raw)[Q], const Geometry& g,
+                            const DynDevice<float>* __restrict__ table, const DynDevice<float>& bulk, int kind_lo,
+                            int kind_hi, int id_lo, int id_hi, uint32_t n_lo, uint32_t n_hi, bool count_hi,
+                            StatAcc& acc)
+{
+  using L = Lattice<Q>;
+  using P = Pair<S>;
+  using T = typename P::T;
+  constexpr bool kForced = KIND == K_FORCED_BGK || KIND == K_FORCED_TRT;
+  // the table entries (nullptr: the bulk entry, the kernel argument)
+  const DynDevice<float>* pe_lo = MASKED && id_lo != kBoxCell ? table + id_lo : nullptr;
+  const DynDevice<float>* pe_hi = MASKED && id_hi != kBoxCell ? table + id_hi : nullptr;
+  const bool field = kForced && g.force != nullptr;
+  // the cell's FORCE when the lattice has a force field (Guo-forced
+  // dynamics; loaded here, after the populations)
+  auto load_force = [&](uint32_t nn, float (&fc)[3]) {
+    const float* __restrict__ F = static_cast<const float*>(g.force);
+    fc[0] = __ldg(F + nn);
+    fc[1] = __ldg(F + size_t(g.stride) + nn);
+    fc[2] = __ldg(F + 2 * size_t(g.stride) + nn);
+  };
+#ifndef OLB_B200_EXACT
+  // both cells go through the two-lane collision unless one is a moving wall
+  // (a pair of two bounce-back walls stores nothing)
+  bool both = true;
+  int lane_lo = kLaneFluid, lane_hi = kLaneFluid;
+  if constexpr (MASKED) {
+    auto mode = [](int kind) {
+      return kind == KIND ? kLaneFluid : (kind == K_BOUNCE_BACK ? kLaneWall : kLanePass);
+    };
+    lane_lo = mode(kind_lo);
+    lane_hi = mode(kind_hi);
+    // a moving wall adds its momentum terms: one cell after the other
+    both = kind_lo != K_BOUNCE_BACK_VELOCITY && kind_hi != K_BOUNCE_BACK_VELOCITY;
+  }
+  if (both) {
+    // Both cells at once, in the scaled representation g_i = s_i (f_i - w_i)
+    // of the storage: lane x the low cell, lane y the high one, straight
+    // from and back to the packed pairs (packed FP32 arithmetic); a wall or
+    // pass lane takes the constants that make the collision a bounce-back or
+    // the identity.
+    float2 g2[Q];
+    static_for<0, Q>([&](auto i) { g2[i] = P::to_float2(raw[i]); });
+    ScaledParams<float> lo = scaled_params<KIND>(pe_lo, MASKED && !g.uniform, bulk, lane_lo);
+    ScaledParams<float> hi = scaled_params<KIND>(pe_hi, MASKED && !g.uniform, bulk, lane_hi);
+    if constexpr (kForced) {
+      if (field) {
+        if (lane_lo == kLaneFluid) load_force(n_lo, lo.force);
+        if (lane_hi == kLaneFluid) load_force(n_hi, hi.force);
+      }
+    }
+    const ScaledParams<float2> q2 = zip_params(lo, hi);
+    float2 r2, u22;
+    collide_scaled<L, KIND>(g2, q2, r2, u22);
+    static_for<0, Q>([&](auto i) { raw[i] = P::from_float2(g2[i]); });
+    if constexpr (STATS) {
+      if (lane_lo == kLaneFluid) acc.add(double(r2.x), double(u22.x));
+      if (lane_hi == kLaneFluid && count_hi) acc.add(double(r2.y), double(u22.y));
+    }
+  } else
+#endif
+  {
+  // One cell after the other (a pair with a wall or boundary cell, and the
+  // exact build).  BGK and TRT cells collide on g directly (collide_scaled);
+  // any other dynamics decodes f_i = g_i / s_i, collides and re-encodes.
+  // s_i of a population equals that of its opposite, so the column read or
+  // written (i or opp(i)) does not change the scale.
+  // the low cell's results wait in packed pairs of populations (half the
+  // registers); the high cell's are packed the same way and the two are
+  // merged with one byte permutation per population
+  constexpr int QP = (Q + 1) / 2;
+  T lo_pack[QP];
+  auto cell = [&](auto half_tag, int kind, const DynDevice<float>* pe) {
+    constexpr bool HI = decltype(half_tag)::value;
+    float gout[Q];
+    static_for<0, Q>([&](auto i) {
+      const float2 fv = P::to_float2(raw[i]);
+      gout[i] = HI ? fv.y : fv.x;
+    });
+    float r = 0.f, u2 = 0.f;
+    bool counted = false, done = false;
+    float fcell[3] = {0.f, 0.f, 0.f};
+    if constexpr (kForced) {
+      if (field && (!MASKED || kind == KIND)) load_force(HI ? n_hi : n_lo, fcell);
+    }
+#ifndef OLB_B200_EXACT
+    if (!MASKED || kind == KIND) {
+      ScaledParams<float> q = scaled_params<KIND>(pe, MASKED && !g.uniform, bulk);
+      if (field) {
+        q.force[0] = fcell[0]; q.force[1] = fcell[1]; q.force[2] = fcell[2];
+      }
+      collide_scaled<L, KIND>(gout, q, r, u2);
+      counted = true;
+      done = true;
+    }
+#endif
+    if (!done) {
+      static_for<0, Q>([&](auto i) {
+        constexpr float inv = 1.f / storage_scale<L>(i);
+        gout[i] *= inv;
+      });
+      counted = collide_any<L, KIND, MASKED>(gout, kind, pe, bulk, fcell, field, g.uniform != 0, r, u2);
+      static_for<0, Q>([&](auto i) {
+        constexpr float sc = storage_scale<L>(i);
+        gout[i] *= sc;
+      });
+    }
+    static_for<0, QP>([&](auto jj) {
+      constexpr int a = 2 * jj.value;
+      constexpr int b = a + 1 < Q ? a + 1 : a;
+      const T packed = P::from_floats(gout[a], gout[b]);
+      if constexpr (!HI) {
+        lo_pack[jj] = packed;
+      } else {
+        raw[a] = pair_perm(lo_pack[jj], packed, 0x5410u);
+        if constexpr (a + 1 < Q) {
+          raw[a + 1] = pair_perm(lo_pack[jj], packed, 0x7632u);
+        }
+      }
+    });
+    if constexpr (STATS) {
+      if (counted && (!HI || count_hi)) acc.add(double(r), double(u2));
+    }
+  };
+  cell(std::integral_constant<bool, false>{}, kind_lo, pe_lo);
+  cell(std::integral_constant<bool, true>{}, kind_hi, pe_hi);
+  }
+}
+
 // One tile of the paired step: the CPT elements (x', y[k], z[k]) of this
 // thread (none where y[k] = ny), each the two cells x' and x' + nx/2.  Masked lattices pass the
 // table entries of both cells (loaded a tile ahead); unmasked ones use `bulk`.
@@ -680,7 +823,6 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
   using L = Lattice<Q>;
   using P = Pair<S>;
   using T = typename P::T;
-  constexpr bool kForced = KIND == K_FORCED_BGK || KIND == K_FORCED_TRT;
   T* __restrict__ pops = reinterpret_cast<T*>(pops_scalar);
   const uint32_t pstride = g.stride >> 1;  // elements per column
 
@@ -730,126 +872,9 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
 
   static_for<0, CPT>([&](auto k) {
     if (!go[k]) return;
-    // the table entries (nullptr: the bulk entry, the kernel argument)
-    const DynDevice<float>* pe_lo = MASKED && id_lo[k] != kBoxCell ? table + id_lo[k] : nullptr;
-    const DynDevice<float>* pe_hi = MASKED && id_hi[k] != kBoxCell ? table + id_hi[k] : nullptr;
-    const bool field = kForced && g.force != nullptr;
-    // the cell's FORCE when the lattice has a force field (Guo-forced
-    // dynamics; loaded here, after the populations)
-    auto load_force = [&](int x, float (&fc)[3]) {
-      const float* __restrict__ F = static_cast<const float*>(g.force);
-      const uint32_t nn = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k]);
-      fc[0] = __ldg(F + nn);
-      fc[1] = __ldg(F + size_t(g.stride) + nn);
-      fc[2] = __ldg(F + 2 * size_t(g.stride) + nn);
-    };
-#ifndef OLB_B200_EXACT
-    // both cells go through the two-lane collision unless one is a moving wall
-    // (a pair of two bounce-back walls stores nothing)
-    bool both = true;
-    int lane_lo = kLaneFluid, lane_hi = kLaneFluid;
-    if constexpr (MASKED) {
-      auto mode = [](int kind) {
-        return kind == KIND ? kLaneFluid : (kind == K_BOUNCE_BACK ? kLaneWall : kLanePass);
-      };
-      lane_lo = mode(kind_lo[k]);
-      lane_hi = mode(kind_hi[k]);
-      // a moving wall adds its momentum terms: one cell after the other
-      both = kind_lo[k] != K_BOUNCE_BACK_VELOCITY && kind_hi[k] != K_BOUNCE_BACK_VELOCITY;
-    }
-    if (both) {
-      // Both cells at once, in the scaled representation g_i = s_i (f_i - w_i)
-      // of the storage: lane x the low cell, lane y the high one, straight
-      // from and back to the packed pairs (packed FP32 arithmetic); a wall or
-      // pass lane takes the constants that make the collision a bounce-back or
-      // the identity.
-      float2 g2[Q];
-      static_for<0, Q>([&](auto i) { g2[i] = P::to_float2(raw[k][i]); });
-      ScaledParams<float> lo = scaled_params<KIND>(pe_lo, MASKED && !g.uniform, bulk, lane_lo);
-      ScaledParams<float> hi = scaled_params<KIND>(pe_hi, MASKED && !g.uniform, bulk, lane_hi);
-      if constexpr (kForced) {
-        if (field) {
-          if (lane_lo == kLaneFluid) load_force(xp, lo.force);
-          if (lane_hi == kLaneFluid) load_force(xp + (g.nx >> 1), hi.force);
-        }
-      }
-      const ScaledParams<float2> q2 = zip_params(lo, hi);
-      float2 r2, u22;
-      collide_scaled<L, KIND>(g2, q2, r2, u22);
-      static_for<0, Q>([&](auto i) { raw[k][i] = P::from_float2(g2[i]); });
-      if constexpr (STATS) {
-        if (lane_lo == kLaneFluid) acc.add(double(r2.x), double(u22.x));
-        if (lane_hi == kLaneFluid) acc.add(double(r2.y), double(u22.y));
-      }
-    } else
-#endif
-    {
-    // One cell after the other (a pair with a wall or boundary cell, and the
-    // exact build).  BGK and TRT cells collide on g directly (collide_scaled);
-    // any other dynamics decodes f_i = g_i / s_i, collides and re-encodes.
-    // s_i of a population equals that of its opposite, so the column read or
-    // written (i or opp(i)) does not change the scale.
-    // the low cell's results wait in packed pairs of populations (half the
-    // registers); the high cell's are packed the same way and the two are
-    // merged with one byte permutation per population
-    constexpr int QP = (Q + 1) / 2;
-    T lo_pack[QP];
-    auto cell = [&](auto half_tag, int kind, const DynDevice<float>* pe) {
-      constexpr bool HI = decltype(half_tag)::value;
-      const int x = HI ? xp + (g.nx >> 1) : xp;
-      float gout[Q];
-      static_for<0, Q>([&](auto i) {
-        const float2 fv = P::to_float2(raw[k][i]);
-        gout[i] = HI ? fv.y : fv.x;
-      });
-      float r = 0.f, u2 = 0.f;
-      bool counted = false, done = false;
-      float fcell[3] = {0.f, 0.f, 0.f};
-      if constexpr (kForced) {
-        if (field && (!MASKED || kind == KIND)) load_force(x, fcell);
-      }
-#ifndef OLB_B200_EXACT
-      if (!MASKED || kind == KIND) {
-        ScaledParams<float> q = scaled_params<KIND>(pe, MASKED && !g.uniform, bulk);
-        if (field) {
-          q.force[0] = fcell[0]; q.force[1] = fcell[1]; q.force[2] = fcell[2];
-        }
-        collide_scaled<L, KIND>(gout, q, r, u2);
-        counted = true;
-        done = true;
-      }
-#endif
-      if (!done) {
-        static_for<0, Q>([&](auto i) {
-          constexpr float inv = 1.f / storage_scale<L>(i);
-          gout[i] *= inv;
-        });
-        counted = collide_any<L, KIND, MASKED>(gout, kind, pe, bulk, fcell, field, g.uniform != 0, r, u2);
-        static_for<0, Q>([&](auto i) {
-          constexpr float sc = storage_scale<L>(i);
-          gout[i] *= sc;
-        });
-      }
-      static_for<0, QP>([&](auto jj) {
-        constexpr int a = 2 * jj.value;
-        constexpr int b = a + 1 < Q ? a + 1 : a;
-        const T packed = P::from_floats(gout[a], gout[b]);
-        if constexpr (!HI) {
-          lo_pack[jj] = packed;
-        } else {
-          raw[k][a] = pair_perm(lo_pack[jj], packed, 0x5410u);
-          if constexpr (a + 1 < Q) {
-            raw[k][a + 1] = pair_perm(lo_pack[jj], packed, 0x7632u);
-          }
-        }
-      });
-      if constexpr (STATS) {
-        if (counted) acc.add(double(r), double(u2));
-      }
-    };
-    cell(std::integral_constant<bool, false>{}, kind_lo[k], pe_lo);
-    cell(std::integral_constant<bool, true>{}, kind_hi[k], pe_hi);
-    }
+    const uint32_t at = (uint32_t(xp) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k]);
+    collide_packed<Q, S, KIND, MASKED, STATS>(raw[k], g, table, bulk, kind_lo[k], kind_hi[k], id_lo[k], id_hi[k], at,
+                                              at + uint32_t(g.nx >> 1) * uint32_t(g.ny) * uint32_t(g.nz), true, acc);
     // recomputed after the collision rather than kept live through it
     PairNeighbours nb(g, int(opaque(uint32_t(xp))), int(opaque(uint32_t(y[k]))), int(opaque(uint32_t(z[k]))));
     const uint32_t ps = opaque(pstride);
@@ -868,6 +893,98 @@ OLB_DEV void paired_tile(S* __restrict__ pops_scalar, const Geometry& g, const D
       }
     });
   });
+}
+
+// ---------------------------------------------------------------------------
+// the step kernel on the natural 16-bit layout (caller-owned buffers, odd nx)
+// Bounded by memory latency: a warp's access moves 64 bytes, half of what the
+// paired layout moves, so bytes in flight are short.  One cell per thread
+// (f_i decoded, collided, encoded) reached 3.67 TB/s on a 191x173x150 D3Q27
+// BF16 box (146 us per step) and 3.87 TB/s on 257^3 D3Q19 FP16 (330 us); two
+// cells per thread, collided together as in the paired kernel, 4.39 TB/s
+// (122 us) and 4.6 TB/s (280 us).  80 registers (3 blocks of 256 per SM) beat
+// 64 where the cells are masked or forced (131x95x122 forced TRT: 33 us
+// against 37) and are even elsewhere.
+//
+// Each thread updates two cells of a plane, one of each of the block's two
+// runs (tile_cells), as the two lanes of the packed collision.  The cells'
+// populations are separate 16-bit accesses, so nothing is asked of their
+// alignment.
+template <int Q, class S, int KIND, bool ODD, bool MASKED, bool STATS>
+OLB_DEV void split_tile(S* __restrict__ pops, const Geometry& g, const DynDevice<float>* __restrict__ table,
+                        const DynDevice<float>& bulk, int x, int (&y)[2], int (&z)[2], int (&id)[2], StatAcc& acc)
+{
+  using L = Lattice<Q>;
+  using T = typename Pair<S>::T;
+  if (y[0] >= g.ny) return;
+  // a missing second cell (the plane's last run) repeats the first, unstored
+  const bool two = y[1] < g.ny;
+  if (!two) {
+    y[1] = y[0];
+    z[1] = z[0];
+    id[1] = id[0];
+  }
+  uint32_t n[2];
+  static_for<0, 2>([&](auto k) {
+    n[k] = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y[k])) * uint32_t(g.nz) + uint32_t(z[k]);
+  });
+  T raw[Q];
+  {
+    const Neighbours a(g, x, y[0], z[0]), b(g, x, y[1], z[1]);
+    static_for<0, Q>([&](auto i) {
+      constexpr int col = ODD ? L::opp(i) : i.value;
+      const S* __restrict__ p = pops + size_t(col) * g.stride;
+      if constexpr (!ODD) {
+        raw[i] = T(p[n[0]], p[n[1]]);
+      } else {
+        raw[i] = T(p[a.template at<-L::c(i, 0), -L::c(i, 1), -L::c(i, 2)>()],
+                   p[b.template at<-L::c(i, 0), -L::c(i, 1), -L::c(i, 2)>()]);
+      }
+    });
+  }
+  int kind[2] = {KIND, KIND};
+  bool store[2] = {true, two};
+  if constexpr (MASKED) {
+    static_for<0, 2>([&](auto k) {
+      if (id[k] != kBoxCell) kind[k] = __ldg(&table[id[k]].kind);
+      store[k] = store[k] && kind[k] != K_BOUNCE_BACK;  // a bounce-back cell's update is a no-op
+    });
+    if (!store[0] && !store[1]) return;
+  }
+  collide_packed<Q, S, KIND, MASKED, STATS>(raw, g, table, bulk, kind[0], kind[1], id[0], id[1], n[0], n[1], two, acc);
+  const Neighbours a(g, int(opaque(uint32_t(x))), int(opaque(uint32_t(y[0]))), int(opaque(uint32_t(z[0])))),
+    b(g, int(opaque(uint32_t(x))), int(opaque(uint32_t(y[1]))), int(opaque(uint32_t(z[1]))));
+  const uint32_t stride = opaque(g.stride);
+  const uint32_t n0 = opaque(n[0]), n1 = opaque(n[1]);
+  static_for<0, Q>([&](auto i) {
+    constexpr int col = ODD ? i.value : L::opp(i);
+    S* __restrict__ p = pops + size_t(col) * stride;
+    uint32_t to0 = n0, to1 = n1;
+    if constexpr (ODD) {
+      to0 = a.template at<L::c(i, 0), L::c(i, 1), L::c(i, 2)>();
+      to1 = b.template at<L::c(i, 0), L::c(i, 1), L::c(i, 2)>();
+    }
+    if (store[0]) p[to0] = raw[i].x;
+    if (store[1]) p[to1] = raw[i].y;
+  });
+}
+
+// MASKED = false takes no ids or table (nullptr)
+template <int Q, class S, int KIND, bool ODD, bool MASKED, bool STATS>
+__global__ void __launch_bounds__(kStepThreads, kSplitMinBlocks)
+aa_step_split_kernel(S* __restrict__ pops, const Geometry g, const uint8_t* __restrict__ ids,
+                     const DynDevice<float>* __restrict__ table, const DynDevice<float> bulk,
+                     StatPartial* __restrict__ partials)
+{
+  const int x = blockIdx.z;
+  int y[2], z[2], id[2] = {};
+  tile_cells(g, y, z);
+  if constexpr (MASKED) load_tile_ids(id, g, ids, x, y, z);
+  StatAcc acc;
+  split_tile<Q, S, KIND, ODD, MASKED, STATS>(pops, g, table, bulk, x, y, z, id, acc);
+  if constexpr (STATS) {
+    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
+  }
 }
 
 template <int Q, class S, int KIND, bool ODD, bool STATS, int CPT, int MINB>
@@ -1491,10 +1608,16 @@ inline dim3 step_grid(const Geometry& g, int bz, int by, int cells_per_thread)
 // 302: the division by nz on an issue-bound kernel) and keeps rectangles.
 inline bool use_flat_tiles(const Geometry& g, int bytes, int bz, int by, int cells_per_thread)
 {
-  if (bytes > 2) return true;
+  if (bytes > 2 || (!g.paired && kSplitNatural16)) return true;
   const uint64_t rows = uint64_t(by) * uint64_t(cells_per_thread);
   const uint64_t lanes = (uint64_t(g.nz) + bz - 1) / bz * bz * ((uint64_t(g.ny) + rows - 1) / rows * rows);
   return 100 * uint64_t(g.ny) * uint64_t(g.nz) < 97 * lanes;
+}
+
+// Cells per thread of the step kernel that serves a lattice.
+inline int step_cells(const Geometry& g, int bytes, int variant)
+{
+  return bytes == 2 && !g.paired && kSplitNatural16 ? 2 : step_variant(bytes, variant).cells_per_thread;
 }
 
 inline dim3 step_block(const Geometry& g, int bz, int by)

@@ -14,7 +14,7 @@ template <int Q, class S, class R, int KIND, int CPT, int MINB>
 static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool masked, bool stats)
 {
   const dim3 block = step_block(a.g, a.block_z, a.block_y);
-  const dim3 grid = step_grid(a.g, a.block_z, a.block_y, CPT);
+  const dim3 grid = step_grid(a.g, a.block_z, a.block_y, step_cells(a.g, int(sizeof(S)), a.variant));
   S* pops = static_cast<S*>(a.pops);
   const DynDevice<R>* table = static_cast<const DynDevice<R>*>(a.table);
   const DynDevice<R>& bulk = *static_cast<const DynDevice<R>*>(a.bulk);
@@ -29,6 +29,10 @@ static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool maske
         break;                                                                                     \
       }                                                                                            \
     }                                                                                              \
+    if constexpr (kHalf && kSplitNatural16) {                                                      \
+      aa_step_split_kernel<Q, S, KIND, O, true, ST><<<grid, block, 0, a.stream>>>(                 \
+        pops, a.g, a.ids, table, bulk, a.partials);                                                \
+    } else                                                                                         \
     aa_step_masked_kernel<Q, S, R, KIND, O, ST, CPT, MINB><<<grid, block, 0, a.stream>>>(          \
       pops, a.g, a.ids, table, bulk, a.partials);                                                  \
   } while (0)
@@ -48,6 +52,10 @@ static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool maske
         break;                                                                                     \
       }                                                                                            \
     }                                                                                              \
+    if constexpr (kHalf && kSplitNatural16) {                                                      \
+      aa_step_split_kernel<Q, S, KIND, O, false, ST><<<grid, block, 0, a.stream>>>(                \
+        pops, a.g, nullptr, nullptr, bulk, a.partials);                                            \
+    } else                                                                                         \
     aa_step_kernel<Q, S, R, KIND, O, ST, CPT, MINB><<<grid, block, 0, a.stream>>>(pops, a.g, bulk, a.partials); \
   } while (0)
     if (odd) {

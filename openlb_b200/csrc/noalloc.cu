@@ -150,7 +150,7 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   // the limit above is the documented one; flat tiles need no more blocks
   if (use_flat_tiles(g, elem, bz, by, cells_per_thread)) {
     set_flat(g);
-    const dim3 grid = step_grid(g, bz, by, cells_per_thread);
+    const dim3 grid = step_grid(g, bz, by, step_cells(g, elem, variant));
     blocks = size_t(grid.x) * grid.y * grid.z;
   }
 

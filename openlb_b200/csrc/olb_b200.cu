@@ -331,14 +331,15 @@ int default_variant(const olb_b200_lattice* L)
 
 int cells_per_thread(const olb_b200_lattice* L)
 {
-  return step_variant(int(L->elem), L->variant).cells_per_thread;
+  return step_cells(L->g, int(L->elem), L->variant);
 }
 
 // How the step kernels cut a plane: as fixed, else by use_flat_tiles.
 void choose_tiles(olb_b200_lattice* L)
 {
   L->g.flat = 0;
-  const bool flat = L->shape_fixed ? L->flat_fixed
+  const bool only_flat = L->elem == 2 && !L->g.paired && kSplitNatural16;
+  const bool flat = only_flat || L->shape_fixed ? only_flat || L->flat_fixed
                                    : use_flat_tiles(L->g, int(L->elem), L->block_z, L->block_y, cells_per_thread(L));
   if (flat) set_flat(L->g);
 }
@@ -1320,7 +1321,7 @@ olb_b200_status olb_b200_get_tuning(olb_b200_lattice* L, olb_b200_tuning* out)
 {
   if (!L || !out) return fail(OLB_B200_ERR_ARG, "get_tuning: null argument");
   out->variant = L->variant;
-  out->cells_per_thread = step_variant(int(L->elem), L->variant).cells_per_thread;
+  out->cells_per_thread = cells_per_thread(L);
   out->min_blocks_per_sm = step_variant(int(L->elem), L->variant).min_blocks;
   out->block_z = L->block_z;
   out->block_y = L->block_y;
@@ -1373,6 +1374,7 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
         L->block_z = bz;
         L->block_y = kStepThreads / bz;
         L->g.flat = 0;
+        if (L->elem == 2 && !L->g.paired && kSplitNatural16) continue;  // flat tiles only
       }
       st = enqueue_steps(L, 2, false);  // warm-up
       if (st != OLB_B200_OK) break;

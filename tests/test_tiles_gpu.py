@@ -1,0 +1,124 @@
+"""Step-kernel tiling, the two-cell kernel of the natural 16-bit layout, the
+statistics reduction and chained launches, at the sizes where they change over:
+planes smaller than a block, exactly a block, one cell more; block counts on
+both sides of the in-kernel reduction."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import openlb_b200 as ob
+from oracle import oracle as O
+from tests import cases as C
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 4
+# 16-bit storage rounds every stored deviation once per step, by at most half a
+# unit in the last place (2^-11 FP16, 2^-8 BF16 relative); the collision spreads
+# that over the other populations with weights summing to at most |1 - omega| +
+# omega < 4: errors stay below 4 * steps roundings of the largest deviation.
+UNIT = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8}
+
+
+def advance(case, f0, steps, storage, shape=None):
+    with ob.Lattice(case.q, case.size, case.periodic, storage=storage) as lat:
+        lat.set_dynamics(C.to_abi_table(case), case.dyn_id)
+        if shape:
+            lat.set_launch_shape(*shape)
+        lat.set_populations(f0)
+        lat.collide_and_stream(steps)
+        return lat.get_populations()
+
+
+def check(case, f0, got, storage):
+    ref = f0.copy()
+    O.step(case, ref, STEPS)
+    if storage in UNIT:
+        valid = ~np.isnan(ref)
+        bound = 4 * STEPS * UNIT[storage] * max(np.abs(f0).max(), np.abs(ref[valid]).max())
+        assert np.abs(got - ref)[valid].max() <= bound
+    else:
+        rel, _ = C.pop_tolerance_violation(case.q, got, ref, 1e-5)
+        assert rel <= 1e-5, rel
+
+
+# planes (ny * nz) of 1, 63, 64, 65, 128, 129, 255, 256, 257, 513 cells
+PLANES = [(1, 1), (7, 9), (4, 16), (5, 13), (8, 16), (3, 43), (5, 51), (16, 16), (257, 1), (19, 27)]
+
+
+@pytest.mark.parametrize("storage,nx", [("f32", 3), ("f16", 4), ("f16", 3), ("bf16", 5)])
+@pytest.mark.parametrize("plane", PLANES)
+def test_periodic_planes_around_a_block(storage, nx, plane):
+    rng = np.random.default_rng(31 + plane[0])
+    case = C.periodic_case(19, (nx,) + plane, kind=O.FORCED_TRT)
+    f0 = C.random_state(19, case.n, np.float32, rng)
+    check(case, f0, advance(case, f0, STEPS, storage), storage)
+
+
+@pytest.mark.parametrize("q,storage,nx", [(19, "f16", 5), (27, "bf16", 5), (19, "f16", 6), (19, "f32", 5)])
+@pytest.mark.parametrize("plane", [(7, 9), (3, 43), (16, 16), (9, 57)])
+def test_cavity_planes_around_a_block(q, storage, nx, plane):
+    rng = np.random.default_rng(57 + plane[1])
+    case = C.cavity_case(q, (nx,) + plane)
+    f0 = C.random_state(q, case.n, np.float32, rng, amp_u=0.01)
+    # slots fed from outside the box hold what the wrap brings; only walls read them
+    check(case, f0, advance(case, f0, STEPS, storage), storage)
+
+
+def test_flat_tiles_and_rectangles_agree():
+    """The same instantiation cut either way: bit for bit."""
+    rng = np.random.default_rng(3)
+    for case in (C.periodic_case(19, (6, 21, 37)), C.cavity_case(19, (6, 21, 37))):
+        f0 = C.random_state(19, case.n, np.float32, rng, amp_u=0.01)
+        flat = advance(case, f0, 5, "f32")
+        for shape in ((32, 8), (64, 4), (32, 1)):
+            assert np.array_equal(flat, advance(case, f0, 5, "f32", shape), equal_nan=True)
+
+
+# one block per plane: 1024 blocks reduce in the step kernel, 1025 and 4099 in a
+# kernel of their own (2 and 5 blocks)
+@pytest.mark.parametrize("nx", [7, 1024, 1025, 4099])
+def test_statistics_around_the_in_kernel_reduction(nx):
+    rng = np.random.default_rng(nx)
+    case = C.periodic_case(19, (nx, 16, 16))
+    f0 = C.random_state(19, case.n, np.float32, rng)
+    with ob.Lattice(19, case.size, case.periodic) as lat:
+        lat.set_dynamics(C.to_abi_table(case))
+        lat.set_step_variant(1)  # one cell per thread
+        lat.set_populations(f0)
+        for _ in range(3):  # again: the reduction leaves its counters as it found them
+            rho, u = (a.astype(np.float64) for a in lat.get_moments())
+            st = lat.collide_and_stream(1, stats=True)
+            u2 = (u * u).sum(0)
+            assert st["n_cells"] == case.n and st["n_nonfinite"] == 0
+            # per-cell values are FP32 (2^-24 relative, a few operations each), their sums FP64
+            np.testing.assert_allclose(st["sum_rho"], rho.sum(), rtol=1e-6)
+            np.testing.assert_allclose(st["sum_usqr"], u2.sum(), rtol=1e-5)
+            np.testing.assert_allclose(st["max_usqr"], u2.max(), rtol=1e-5)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("boundary", [False, True])
+def test_chained_steps_equal_separate_steps(storage, boundary):
+    """Launches that overlap their predecessor's end give what launches with a
+    synchronisation between them give, bit for bit."""
+    rng = np.random.default_rng(12)
+    case = (C.interpolated_channel_case(19, (14, 12, 10)) if boundary else C.cavity_case(19, (14, 12, 10)))
+    f0 = C.random_state(19, case.n, np.float32, rng, amp_u=0.01)
+    out = []
+    for together in (True, False):
+        with ob.Lattice(19, case.size, case.periodic, storage=storage) as lat:
+            lat.set_dynamics(C.to_abi_table(case), case.dyn_id)
+            if boundary:
+                lat.set_boundary_values(*C.boundary_cells_and_values(case))
+                lat.set_boundary_noise(0.02, 5)
+            lat.set_populations(f0)
+            if together:
+                lat.collide_and_stream(60)
+            else:
+                for _ in range(60):
+                    lat.collide_and_stream(1)
+                    lat.synchronize()
+            out.append(lat.get_populations())
+    assert np.array_equal(out[0], out[1], equal_nan=True)
