@@ -46,8 +46,8 @@ struct Geometry {
   // the bulk entry's constants, so the step kernel takes them from the kernel
   // argument instead of loading them from the cell's table entry
   int32_t uniform;
-  // flat tiles of the step kernels: 0 or the multiplier and shift of
-  // floor(n / nz) = (mulhi(n, flat_mul) + n) >> flat_shift (tile_cells)
+  // flat tiles of the step kernels (tile_cells): 0 or the threads of a block,
+  // with floor(n / nz) = (mulhi(n, flat_mul) + n) >> flat_shift
   int32_t flat;
   uint32_t flat_mul, flat_shift;
 };
@@ -266,7 +266,7 @@ struct StatAcc {
 // The (y, z) of this thread's CPT cells.  Two ways to cut a plane x into blocks:
 //   rectangles  blockDim.x cells along z by blockDim.y * CPT rows (the launch
 //               shape); lanes beyond nz and rows beyond ny idle;
-//   flat        CPT runs of kStepThreads consecutive cells of the plane's
+//   flat        CPT runs of g.flat (the block size) consecutive cells of the plane's
 //               index y*nz + z, so every lane but the plane's last few has a
 //               cell, whatever nz and ny; y costs one multiply-high
 //               (Granlund & Montgomery, PLDI 1994).
@@ -283,7 +283,7 @@ OLB_DEV void tile_cells(const Geometry& g, int (&y)[CPT], int (&z)[CPT])
 {
   if (g.flat) {
     static_for<0, CPT>([&](auto k) {
-      const uint32_t n = (blockIdx.x * uint32_t(CPT) + uint32_t(k.value)) * uint32_t(kStepThreads) + threadIdx.x;
+      const uint32_t n = (blockIdx.x * uint32_t(CPT) + uint32_t(k.value)) * uint32_t(g.flat) + threadIdx.x;
       flat_cell(g, n, y[k], z[k]);
     });
   } else {
@@ -1591,28 +1591,28 @@ inline dim3 step_grid(const Geometry& g, int bz, int by, int cells_per_thread)
 {
   const unsigned planes = unsigned(g.paired ? g.nx / 2 : g.nx);
   if (g.flat) {
-    const uint64_t tile = uint64_t(kStepThreads) * uint64_t(cells_per_thread);
+    const uint64_t tile = uint64_t(g.flat) * uint64_t(cells_per_thread);
     return dim3(unsigned((uint64_t(g.ny) * uint64_t(g.nz) + tile - 1) / tile), 1, planes);
   }
   const int rows = by * cells_per_thread;
   return dim3((g.nz + bz - 1) / bz, (g.ny + rows - 1) / rows, planes);
 }
 
-// Whether an unfixed launch shape gives way to flat tiles.  Rectangles leave
-// lanes without cells when nz or ny is no multiple of theirs: 0.58 of the lanes
-// have cells at 191x173x150, and flat tiles take 125 us against 144 (cavity,
-// FP32), 31 against 35 at 200x120x100 (FP16, 0.78 of the lanes), 12.3 against
-// 15.4 at 97x61x75.  With every lane busy (256^3) FP32 and FP64 still gain
-// 0.1 % to 3 % (389 us against 402: a block's loads are one contiguous run of
-// every column), 16-bit storage loses 1 % to 3 % (D3Q27 BF16 312 us against
-// 302: the division by nz on an issue-bound kernel) and keeps rectangles.
-inline bool use_flat_tiles(const Geometry& g, int bytes, int bz, int by, int cells_per_thread)
-{
-  if (bytes > 2 || (!g.paired && kSplitNatural16)) return true;
-  const uint64_t rows = uint64_t(by) * uint64_t(cells_per_thread);
-  const uint64_t lanes = (uint64_t(g.nz) + bz - 1) / bz * bz * ((uint64_t(g.ny) + rows - 1) / rows * rows);
-  return 100 * uint64_t(g.ny) * uint64_t(g.nz) < 97 * lanes;
-}
+// Threads of a block of flat tiles, which every lattice takes unless the caller
+// or the autotuner has fixed a launch shape.
+//   Against rectangles: those leave lanes without cells when nz or ny is no
+// multiple of theirs (0.58 of the lanes have cells at 191x173x150: 144 us
+// against 125 with flat tiles for an FP32 cavity; 35 against 31 at 200x120x100
+// FP16; 15.4 against 12.3 at 97x61x75), and at 256^3, where every lane is busy,
+// flat tiles still gain 0.1 % to 3 % (FP32 402 us against 389: a block's loads
+// are one contiguous run of every column).
+//   Block size: the 16-bit kernels alternate between waiting for loads and
+// bursts of arithmetic, and the warps of one block do so together; blocks of
+// 64 threads (the same registers and warps per SM) mix the phases better:
+// 256^3 D3Q27 BF16 Smagorinsky 389 -> 372 us (377 with 128 threads), D3Q27 BF16
+// TRT 302 -> 292, D3Q19 FP16 212 -> 206, 384x192x192 FP16 forced TRT 228 -> 217.
+// FP32 gains nothing from it (257^3 cavity 418 against 417 us with 128).
+inline int flat_threads(int bytes) { return bytes == 2 ? 64 : kStepThreads; }
 
 // Cells per thread of the step kernel that serves a lattice.
 inline int step_cells(const Geometry& g, int bytes, int variant)
@@ -1622,15 +1622,15 @@ inline int step_cells(const Geometry& g, int bytes, int variant)
 
 inline dim3 step_block(const Geometry& g, int bz, int by)
 {
-  return g.flat ? dim3(kStepThreads, 1) : dim3(bz, by);
+  return g.flat ? dim3(g.flat, 1) : dim3(bz, by);
 }
 
-// the constants of the flat tiles' division by nz
-inline void set_flat(Geometry& g)
+// flat tiles of `threads` threads and the constants of their division by nz
+inline void set_flat(Geometry& g, int threads)
 {
   uint32_t s = 0;
   while ((uint64_t(1) << s) < uint64_t(g.nz)) ++s;
-  g.flat = 1;
+  g.flat = threads;
   g.flat_mul = uint32_t(((uint64_t(1) << 32) * ((uint64_t(1) << s) - uint64_t(g.nz))) / uint64_t(g.nz) + 1);
   g.flat_shift = s;
 }

@@ -147,12 +147,11 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
              bz, by, blocks, kMaxBlocks);
     return noalloc_fail(OLB_B200_ERR_ARG, buf);
   }
-  // the limit above is the documented one; flat tiles need no more blocks
-  if (use_flat_tiles(g, elem, bz, by, cells_per_thread)) {
-    set_flat(g);
-    const dim3 grid = step_grid(g, bz, by, step_cells(g, elem, variant));
-    blocks = size_t(grid.x) * grid.y * grid.z;
-  }
+  // the limit above is the documented one; flat tiles of kStepThreads, which a
+  // step with statistics takes, need no more blocks
+  set_flat(g, kStepThreads);
+  const dim3 stat_grid = step_grid(g, bz, by, step_cells(g, elem, variant));
+  blocks = size_t(stat_grid.x) * stat_grid.y * stat_grid.z;
 
   cudaError_t e = cudaSetDevice(desc->device);
   if (e != cudaSuccess) return noalloc_cuda(e, "cudaSetDevice");
@@ -174,6 +173,7 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
     StepLaunch a;
     a.pops = device_pops;
     a.g = g;
+    if (!last_stats) a.g.flat = flat_threads(elem);
     a.ids = nullptr;
     a.table = nullptr;
     a.bulk = params;

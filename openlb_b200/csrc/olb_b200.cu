@@ -334,14 +334,22 @@ int cells_per_thread(const olb_b200_lattice* L)
   return step_cells(L->g, int(L->elem), L->variant);
 }
 
-// How the step kernels cut a plane: as fixed, else by use_flat_tiles.
+// How the step kernels cut a plane: flat tiles (flat_threads) unless a launch
+// shape is fixed.
 void choose_tiles(olb_b200_lattice* L)
 {
-  L->g.flat = 0;
   const bool only_flat = L->elem == 2 && !L->g.paired && kSplitNatural16;
-  const bool flat = only_flat || L->shape_fixed ? only_flat || L->flat_fixed
-                                   : use_flat_tiles(L->g, int(L->elem), L->block_z, L->block_y, cells_per_thread(L));
-  if (flat) set_flat(L->g);
+  L->g.flat = 0;
+  if (only_flat || !L->shape_fixed || L->flat_fixed) set_flat(L->g, flat_threads(int(L->elem)));
+}
+
+// The geometry a step launches with.  Steps that reduce statistics use blocks
+// of kStepThreads: the block reduction and its partials cost per block.
+Geometry step_geometry(const olb_b200_lattice* L, bool stats)
+{
+  Geometry g = L->g;
+  if (g.flat && stats) g.flat = kStepThreads;
+  return g;
 }
 
 template <class F>
@@ -372,9 +380,10 @@ size_t boundary_blocks(const olb_b200_lattice* L)
   return (size_t(L->n_bc) + kBoundaryThreads - 1) / kBoundaryThreads;
 }
 
+// blocks of a step that reduces statistics
 size_t step_blocks(const olb_b200_lattice* L)
 {
-  const dim3 grid = step_grid(L->g, L->block_z, L->block_y, cells_per_thread(L));
+  const dim3 grid = step_grid(step_geometry(L, true), L->block_z, L->block_y, cells_per_thread(L));
   return size_t(grid.x) * grid.y * grid.z;
 }
 
@@ -506,7 +515,7 @@ olb_b200_status enqueue_steps(olb_b200_lattice* L, int steps, bool stats_last)
     const bool stats = stats_last && s == steps - 1;
     StepLaunch a;
     a.pops = L->pops;
-    a.g = L->g;
+    a.g = step_geometry(L, stats);
     a.ids = L->masked ? L->ids : nullptr;
     a.table = L->table;
     a.bulk = L->bulk;
@@ -1369,7 +1378,7 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
       L->variant = v;
       if (flat) {
         default_shape(L, L->block_z, L->block_y);
-        set_flat(L->g);
+        set_flat(L->g, flat_threads(int(L->elem)));
       } else {
         L->block_z = bz;
         L->block_y = kStepThreads / bz;
