@@ -101,6 +101,50 @@ struct StatPartial {
   unsigned long long n_nonfinite;
 };
 
+// Scratch of a reduction over several blocks, zero before the first use;
+// `arrived` is zero again after each.
+constexpr int kReduceBlocks = 64;
+struct StatStage {
+  StatPartial part[kReduceBlocks];
+  unsigned arrived;
+};
+
+// a reduced statistic and the number of the reduction that wrote it (written
+// last: a host that reads it from pinned memory waits for its number)
+struct StatResult {
+  StatPartial p;
+  unsigned long long seq;
+};
+
+// Where the blocks of a kernel leave their partials.  With a stage the last
+// block to finish also reduces them into `result`; without, a
+// reduce_partials_kernel does.
+struct StatSink {
+  StatPartial* partials = nullptr;
+  StatStage* stage = nullptr;
+  StatResult* result = nullptr;
+  unsigned long long seq = 0;
+};
+
+// ---------------------------------------------------------------------------
+// launches chained on a stream (programmatic dependent launch)
+//
+// A step of a small lattice takes about as long as a launch: a kernel that lets
+// its successor start (next_may_start, first thing) and waits for its
+// predecessor's results only when it needs them (after_previous) hides the
+// launch and the drain of the last blocks.  Every block of a kernel passes
+// after_previous before it ends, so a finished kernel implies finished
+// predecessors.  The pointer goes through the wait: no load from it can move
+// ahead of it.  In a launch without the attribute both do nothing.
+OLB_DEV void next_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+template <class T>
+OLB_DEV T* after_previous(T* p)
+{
+  asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+  return p;
+}
+
 // ---------------------------------------------------------------------------
 // storage element conversions (plain loads: the array is read and written in
 // place by the same kernel, so the read-only data path is not used)
@@ -177,26 +221,75 @@ OLB_DEV void warp_reduce(double& a, double& b, double& m, unsigned long long& n,
   }
 }
 
-OLB_DEV void block_stats(double a, double b, double m, unsigned long long n, unsigned long long nf,
-                         StatPartial* out)
+// sum over the block's threads (256 or a multiple of 32), valid in thread 0
+OLB_DEV StatPartial block_sum(StatPartial v)
 {
   __shared__ StatPartial warp_part[32];
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
   const int nthreads = blockDim.x * blockDim.y;
-  warp_reduce(a, b, m, n, nf);
+  warp_reduce(v.sum_rho, v.sum_usqr, v.max_usqr, v.n_cells, v.n_nonfinite);
   const int lane = tid & 31, warp = tid >> 5;
   if (lane == 0) {
-    warp_part[warp] = StatPartial{a, b, m, n, nf};
+    warp_part[warp] = v;
   }
   __syncthreads();
   if (warp == 0) {
     const int nw = (nthreads + 31) >> 5;
-    StatPartial p = lane < nw ? warp_part[lane] : StatPartial{0, 0, 0, 0, 0};
-    warp_reduce(p.sum_rho, p.sum_usqr, p.max_usqr, p.n_cells, p.n_nonfinite);
-    if (lane == 0) {
-      const size_t bid = blockIdx.x + size_t(gridDim.x) * (blockIdx.y + size_t(gridDim.y) * blockIdx.z);
-      out[bid] = p;
-    }
+    v = lane < nw ? warp_part[lane] : StatPartial{0, 0, 0, 0, 0};
+    warp_reduce(v.sum_rho, v.sum_usqr, v.max_usqr, v.n_cells, v.n_nonfinite);
+  }
+  return v;
+}
+
+// the block's share of parts[begin, end): a fixed assignment to threads and a
+// fixed tree (deterministic for a given block size); valid in thread 0
+OLB_DEV StatPartial sum_partials(const StatPartial* parts, size_t begin, size_t end)
+{
+  StatPartial v{0, 0, 0, 0, 0};
+  for (size_t k = begin + threadIdx.x + blockDim.x * threadIdx.y; k < end; k += blockDim.x * blockDim.y) {
+    // from L2: other blocks wrote them
+    v.sum_rho += __ldcg(&parts[k].sum_rho);
+    v.sum_usqr += __ldcg(&parts[k].sum_usqr);
+    v.max_usqr = fmax(v.max_usqr, __ldcg(&parts[k].max_usqr));
+    v.n_cells += __ldcg(&parts[k].n_cells);
+    v.n_nonfinite += __ldcg(&parts[k].n_nonfinite);
+  }
+  return block_sum(v);
+}
+
+OLB_DEV void write_result(StatResult* out, const StatPartial& p, unsigned long long seq)
+{
+  out->p = p;
+  __threadfence_system();
+  *reinterpret_cast<volatile unsigned long long*>(&out->seq) = seq;
+}
+
+// true in every thread of the block that arrives last of `blocks`; what the
+// others wrote before arriving is visible to it
+OLB_DEV bool last_to_arrive(unsigned* arrived, unsigned blocks)
+{
+  __shared__ bool last;
+  if (threadIdx.x + threadIdx.y == 0) {
+    __threadfence();
+    last = atomicAdd(arrived, 1u) == blocks - 1;
+    if (last) *arrived = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
+OLB_DEV void block_stats(double a, double b, double m, unsigned long long n, unsigned long long nf,
+                         const StatSink& sink)
+{
+  const StatPartial v = block_sum(StatPartial{a, b, m, n, nf});
+  const unsigned blocks = gridDim.x * gridDim.y * gridDim.z;
+  if (threadIdx.x + threadIdx.y == 0) {
+    sink.partials[blockIdx.x + size_t(gridDim.x) * (blockIdx.y + size_t(gridDim.y) * blockIdx.z)] = v;
+  }
+  if (sink.stage && last_to_arrive(&sink.stage->arrived, blocks)) {
+    const StatPartial sum = sum_partials(sink.partials, 0, blocks);
+    if (threadIdx.x + threadIdx.y == 0) write_result(sink.result, sum, sink.seq);
   }
 }
 
@@ -440,15 +533,17 @@ OLB_DEV void step_tile(S* __restrict__ pops, const Geometry& g, const DynDevice<
 // step_grid().
 template <int Q, class S, class R, int KIND, bool ODD, bool STATS, int CPT, int MINB>
 __global__ void __launch_bounds__(kStepThreads, MINB)
-aa_step_kernel(S* __restrict__ pops, const Geometry g, const DynDevice<R> bulk, StatPartial* __restrict__ partials)
+aa_step_kernel(S* __restrict__ pops, const Geometry g, const DynDevice<R> bulk, const StatSink sink)
 {
+  next_may_start();
   int y[CPT], z[CPT];
   tile_cells(g, y, z);
   const int none[CPT] = {};
   StatAcc acc;
+  pops = after_previous(pops);
   step_tile<Q, S, R, KIND, ODD, false, STATS, CPT>(pops, g, nullptr, bulk, int(blockIdx.z), y, z, none, acc);
   if constexpr (STATS) {
-    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
+    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, sink);
   }
 }
 
@@ -475,16 +570,18 @@ template <int Q, class S, class R, int KIND, bool ODD, bool STATS, int CPT, int 
 __global__ void __launch_bounds__(kStepThreads, MINB)
 aa_step_masked_kernel(S* __restrict__ pops, const Geometry g, const uint8_t* __restrict__ ids,
                       const DynDevice<R>* __restrict__ table, const DynDevice<R> bulk,
-                      StatPartial* __restrict__ partials)
+                      const StatSink sink)
 {
+  next_may_start();
   const int x = blockIdx.z;
   int y[CPT], z[CPT], id[CPT];
   tile_cells(g, y, z);
   load_tile_ids(id, g, ids, x, y, z);
   StatAcc acc;
+  pops = after_previous(pops);
   step_tile<Q, S, R, KIND, ODD, true, STATS, CPT>(pops, g, table, bulk, x, y, z, id, acc);
   if constexpr (STATS) {
-    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
+    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, sink);
   }
 }
 
@@ -974,31 +1071,35 @@ template <int Q, class S, int KIND, bool ODD, bool MASKED, bool STATS>
 __global__ void __launch_bounds__(kStepThreads, kSplitMinBlocks)
 aa_step_split_kernel(S* __restrict__ pops, const Geometry g, const uint8_t* __restrict__ ids,
                      const DynDevice<float>* __restrict__ table, const DynDevice<float> bulk,
-                     StatPartial* __restrict__ partials)
+                     const StatSink sink)
 {
+  next_may_start();
   const int x = blockIdx.z;
   int y[2], z[2], id[2] = {};
   tile_cells(g, y, z);
   if constexpr (MASKED) load_tile_ids(id, g, ids, x, y, z);
   StatAcc acc;
+  pops = after_previous(pops);
   split_tile<Q, S, KIND, ODD, MASKED, STATS>(pops, g, table, bulk, x, y, z, id, acc);
   if constexpr (STATS) {
-    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
+    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, sink);
   }
 }
 
 template <int Q, class S, int KIND, bool ODD, bool STATS, int CPT, int MINB>
 __global__ void __launch_bounds__(kStepThreads, MINB)
 aa_step_paired_kernel(S* __restrict__ pops, const Geometry g, const DynDevice<float> bulk,
-                      StatPartial* __restrict__ partials)
+                      const StatSink sink)
 {
+  next_may_start();
   int y[CPT], z[CPT];
   tile_cells(g, y, z);
   const int none[CPT] = {};
   StatAcc acc;
+  pops = after_previous(pops);
   paired_tile<Q, S, KIND, ODD, false, STATS, CPT>(pops, g, nullptr, bulk, int(blockIdx.z), y, z, none, none, acc);
   if constexpr (STATS) {
-    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
+    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, sink);
   }
 }
 
@@ -1007,23 +1108,27 @@ template <int Q, class S, int KIND, bool ODD, bool STATS, int CPT, int MINB>
 __global__ void __launch_bounds__(kStepThreads, MINB)
 aa_step_masked_paired_kernel(S* __restrict__ pops, const Geometry g, const uint8_t* __restrict__ ids,
                              const DynDevice<float>* __restrict__ table, const DynDevice<float> bulk,
-                             StatPartial* __restrict__ partials)
+                             const StatSink sink)
 {
+  next_may_start();
   const int xp = blockIdx.z;
   int y[CPT], z[CPT], lo[CPT], hi[CPT];
   tile_cells(g, y, z);
   load_tile_ids(lo, g, ids, xp, y, z);
   load_tile_ids(hi, g, ids, xp + (g.nx >> 1), y, z);
   StatAcc acc;
+  pops = after_previous(pops);
   paired_tile<Q, S, KIND, ODD, true, STATS, CPT>(pops, g, table, bulk, xp, y, z, lo, hi, acc);
   if constexpr (STATS) {
-    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, partials);
+    block_stats(acc.rho, acc.usqr, acc.max, acc.n, acc.nf, sink);
   }
 }
 
-// Deterministic second pass over the per-block partials (one block).
-__global__ void reduce_partials_kernel(const StatPartial* __restrict__ parts, size_t count,
-                                       StatPartial* __restrict__ out);
+// Deterministic second pass over the per-block partials: up to kReduceBlocks
+// blocks (one block needs no stage), the last of which adds up the others.
+__global__ void reduce_partials_kernel(const StatPartial* parts, size_t count, StatStage* stage, StatResult* out,
+                                       unsigned long long seq);
+constexpr int kReduceThreads = 256;
 
 // ---------------------------------------------------------------------------
 // logical-layout gather / scatter and moments
@@ -1317,12 +1422,14 @@ OLB_DEV R cell_density(const S* __restrict__ pops, const Geometry& g, bool shift
 
 // pass 1: velocity of every interpolated cell (its momenta, post-stream state)
 template <int Q, class S, class R>
-__global__ void bc_velocity_kernel(const S* __restrict__ pops, const Geometry g, bool shifted,
+__global__ void bc_velocity_kernel(const S* pops, const Geometry g, bool shifted,
                                    const uint8_t* __restrict__ ids, const DynDevice<R>* __restrict__ table,
                                    const uint32_t* __restrict__ cells, uint32_t count)
 {
   using L = Lattice<Q>;
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  next_may_start();
+  pops = after_previous(pops);
   if (k >= count) return;
   const uint32_t n = cells[k];
   int x, y, z;
@@ -1347,6 +1454,8 @@ __global__ void plane_fd_kernel(S* __restrict__ pops, const Geometry g, bool shi
 {
   using L = Lattice<Q>;
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  next_may_start();
+  pops = after_previous(pops);
   if (k >= count) return;
   const uint32_t n = cells[k];
   int x, y, z;
@@ -1410,12 +1519,14 @@ template <int Q, class S, class R, int KIND, bool STATS>
 __global__ void boundary_collide_kernel(S* __restrict__ pops, const Geometry g, bool shifted,
                                         const uint8_t* __restrict__ ids, const DynDevice<R>* __restrict__ table,
                                         const uint32_t* __restrict__ cells, uint32_t count,
-                                        StatPartial* __restrict__ partials)
+                                        const StatSink sink)
 {
   using L = Lattice<Q>;
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   double s_rho = 0., s_usqr = 0., s_max = 0.;
   unsigned long long s_n = 0, s_nf = 0;
+  next_may_start();
+  pops = after_previous(pops);
   if (k < count) {
     const uint32_t n = cells[k];
     int x, y, z;
@@ -1436,7 +1547,7 @@ __global__ void boundary_collide_kernel(S* __restrict__ pops, const Geometry g, 
     }
   }
   if constexpr (STATS) {
-    block_stats(s_rho, s_usqr, s_max, s_n, s_nf, partials);
+    block_stats(s_rho, s_usqr, s_max, s_n, s_nf, sink);
   }
 }
 
@@ -1454,6 +1565,8 @@ __global__ void outer_velocity_kernel(S* __restrict__ pops, const Geometry g, bo
 {
   using L = Lattice<Q>;
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  next_may_start();
+  pops = after_previous(pops);
   if (k >= count) return;
   const uint32_t n = cells[k];
   int x, y, z;
@@ -1540,13 +1653,31 @@ __global__ void outer_velocity_kernel(S* __restrict__ pops, const Geometry g, bo
 // ---------------------------------------------------------------------------
 // host-side launch entry points (explicitly instantiated per lattice/storage)
 
+// Launch whose kernel may start before the stream's previous kernel has ended
+// (it waits by after_previous); an ordinary launch when !chained.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), bool chained, dim3 grid, dim3 block, cudaStream_t stream, A&&... args)
+{
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.stream = stream;
+  config.attrs = &attr;
+  config.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&config, kernel, P(args)...);
+}
+
 struct StepLaunch {
   void* pops;
   Geometry g;
   const uint8_t* ids;      // device, or nullptr
   const void* table;       // device DynDevice<R>[]
   const void* bulk;        // host DynDevice<R>
-  StatPartial* partials;   // device, gridDim product entries
+  StatSink sink;           // partials: gridDim product entries (statistics only)
+  bool chained = false;    // the previous work on the stream may be overlapped (launch_chained)
   int block_z, block_y;
   int variant;             // index into kStepVariants
   cudaStream_t stream;
@@ -1571,11 +1702,11 @@ template <int Q, class S, class R>
 cudaError_t launch_moments(const void* pops, const Geometry& g, bool shifted, const uint8_t* ids,
                            const void* table, void* rho, void* u, cudaStream_t stream);
 
-// the boundary pre-pass over `count` cells; partials == nullptr: no statistics
+// the boundary pre-pass over `count` cells; sink.partials == nullptr: no statistics
 template <int Q, class S, class R>
 cudaError_t launch_boundary_collide(void* pops, const Geometry& g, bool shifted, const uint8_t* ids,
                                     const void* table, int kind, const uint32_t* cells, uint32_t count,
-                                    StatPartial* partials, cudaStream_t stream);
+                                    const StatSink& sink, cudaStream_t stream);
 constexpr int kBoundaryThreads = 128;
 
 // the PostStream passes: cells[0, n_flat) are the interpolated flat cells

@@ -10,8 +10,8 @@
 
 namespace olb_b200 {
 
-template <int Q, class S, class R, int KIND, int CPT, int MINB>
-static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool masked, bool stats)
+template <int Q, class S, class R, int KIND, int CPT, int MINB, bool ODD, bool STATS>
+static cudaError_t launch_step_one(const StepLaunch& a, bool masked)
 {
   const dim3 block = step_block(a.g, a.block_z, a.block_y);
   const dim3 grid = step_grid(a.g, a.block_z, a.block_y, step_cells(a.g, int(sizeof(S)), a.variant));
@@ -19,53 +19,38 @@ static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool maske
   const DynDevice<R>* table = static_cast<const DynDevice<R>*>(a.table);
   const DynDevice<R>& bulk = *static_cast<const DynDevice<R>*>(a.bulk);
   constexpr bool kHalf = std::is_same_v<S, __half> || std::is_same_v<S, __nv_bfloat16>;
-  if (masked) {
-#define OLB_LAUNCH(O, ST)                                                                          \
-  do {                                                                                             \
-    if constexpr (kHalf) {                                                                         \
-      if (a.g.paired) {                                                                            \
-        aa_step_masked_paired_kernel<Q, S, KIND, O, ST, CPT, MINB><<<grid, block, 0, a.stream>>>(  \
-          pops, a.g, a.ids, table, bulk, a.partials);                                              \
-        break;                                                                                     \
-      }                                                                                            \
-    }                                                                                              \
-    if constexpr (kHalf && kSplitNatural16) {                                                      \
-      aa_step_split_kernel<Q, S, KIND, O, true, ST><<<grid, block, 0, a.stream>>>(                 \
-        pops, a.g, a.ids, table, bulk, a.partials);                                                \
-    } else                                                                                         \
-    aa_step_masked_kernel<Q, S, R, KIND, O, ST, CPT, MINB><<<grid, block, 0, a.stream>>>(          \
-      pops, a.g, a.ids, table, bulk, a.partials);                                                  \
-  } while (0)
-    if (odd) {
-      if (stats) OLB_LAUNCH(true, true); else OLB_LAUNCH(true, false);
-    } else {
-      if (stats) OLB_LAUNCH(false, true); else OLB_LAUNCH(false, false);
+  if constexpr (kHalf) {
+    if (a.g.paired) {
+      return masked ? launch_chained(aa_step_masked_paired_kernel<Q, S, KIND, ODD, STATS, CPT, MINB>, a.chained, grid,
+                                     block, a.stream, pops, a.g, a.ids, table, bulk, a.sink)
+                    : launch_chained(aa_step_paired_kernel<Q, S, KIND, ODD, STATS, CPT, MINB>, a.chained, grid, block,
+                                     a.stream, pops, a.g, bulk, a.sink);
     }
-#undef OLB_LAUNCH
-  } else {
-#define OLB_LAUNCH(O, ST)                                                                          \
-  do {                                                                                             \
-    if constexpr (kHalf) {                                                                         \
-      if (a.g.paired) {                                                                            \
-        aa_step_paired_kernel<Q, S, KIND, O, ST, CPT, MINB><<<grid, block, 0, a.stream>>>(         \
-          pops, a.g, bulk, a.partials);                                                            \
-        break;                                                                                     \
-      }                                                                                            \
-    }                                                                                              \
-    if constexpr (kHalf && kSplitNatural16) {                                                      \
-      aa_step_split_kernel<Q, S, KIND, O, false, ST><<<grid, block, 0, a.stream>>>(                \
-        pops, a.g, nullptr, nullptr, bulk, a.partials);                                            \
-    } else                                                                                         \
-    aa_step_kernel<Q, S, R, KIND, O, ST, CPT, MINB><<<grid, block, 0, a.stream>>>(pops, a.g, bulk, a.partials); \
-  } while (0)
-    if (odd) {
-      if (stats) OLB_LAUNCH(true, true); else OLB_LAUNCH(true, false);
-    } else {
-      if (stats) OLB_LAUNCH(false, true); else OLB_LAUNCH(false, false);
+    if constexpr (kSplitNatural16) {
+      return masked ? launch_chained(aa_step_split_kernel<Q, S, KIND, ODD, true, STATS>, a.chained, grid, block,
+                                     a.stream, pops, a.g, a.ids, table, bulk, a.sink)
+                    : launch_chained(aa_step_split_kernel<Q, S, KIND, ODD, false, STATS>, a.chained, grid, block,
+                                     a.stream, pops, a.g, a.ids, table, bulk, a.sink);
     }
-#undef OLB_LAUNCH
   }
-  return cudaGetLastError();
+  if constexpr (!kHalf || !kSplitNatural16) {
+    return masked ? launch_chained(aa_step_masked_kernel<Q, S, R, KIND, ODD, STATS, CPT, MINB>, a.chained, grid, block,
+                                   a.stream, pops, a.g, a.ids, table, bulk, a.sink)
+                  : launch_chained(aa_step_kernel<Q, S, R, KIND, ODD, STATS, CPT, MINB>, a.chained, grid, block,
+                                   a.stream, pops, a.g, bulk, a.sink);
+  }
+  return cudaErrorInvalidValue;
+}
+
+template <int Q, class S, class R, int KIND, int CPT, int MINB>
+static cudaError_t launch_step_variant(const StepLaunch& a, bool odd, bool masked, bool stats)
+{
+  if (odd) {
+    return stats ? launch_step_one<Q, S, R, KIND, CPT, MINB, true, true>(a, masked)
+                 : launch_step_one<Q, S, R, KIND, CPT, MINB, true, false>(a, masked);
+  }
+  return stats ? launch_step_one<Q, S, R, KIND, CPT, MINB, false, true>(a, masked)
+               : launch_step_one<Q, S, R, KIND, CPT, MINB, false, false>(a, masked);
 }
 
 template <int Q, class S, class R, int KIND>
@@ -143,28 +128,24 @@ cudaError_t launch_moments(const void* pops, const Geometry& g, bool shifted, co
 template <int Q, class S, class R>
 cudaError_t launch_boundary_collide(void* pops, const Geometry& g, bool shifted, const uint8_t* ids,
                                     const void* table, int kind, const uint32_t* cells, uint32_t count,
-                                    StatPartial* partials, cudaStream_t stream)
+                                    const StatSink& sink, cudaStream_t stream)
 {
   if (count == 0) return cudaSuccess;
   const unsigned blocks = (count + kBoundaryThreads - 1) / kBoundaryThreads;
   S* p = static_cast<S*>(pops);
   const auto* t = static_cast<const DynDevice<R>*>(table);
 #define OLB_BC_LAUNCH(K)                                                                             \
-  do {                                                                                               \
-    if (partials)                                                                                    \
-      boundary_collide_kernel<Q, S, R, K, true><<<blocks, kBoundaryThreads, 0, stream>>>(            \
-        p, g, shifted, ids, t, cells, count, partials);                                              \
-    else                                                                                             \
-      boundary_collide_kernel<Q, S, R, K, false><<<blocks, kBoundaryThreads, 0, stream>>>(           \
-        p, g, shifted, ids, t, cells, count, partials);                                              \
-  } while (0)
+  return sink.partials                                                                               \
+    ? launch_chained(boundary_collide_kernel<Q, S, R, K, true>, true, blocks, kBoundaryThreads,      \
+                     stream, p, g, shifted, ids, t, cells, count, sink)                              \
+    : launch_chained(boundary_collide_kernel<Q, S, R, K, false>, true, blocks, kBoundaryThreads,     \
+                     stream, p, g, shifted, ids, t, cells, count, sink)
   switch (kind) {
-  case K_TRT: OLB_BC_LAUNCH(K_TRT); break;
-  case K_SMAGORINSKY: OLB_BC_LAUNCH(K_SMAGORINSKY); break;
-  default: OLB_BC_LAUNCH(K_BGK); break;
+  case K_TRT: OLB_BC_LAUNCH(K_TRT);
+  case K_SMAGORINSKY: OLB_BC_LAUNCH(K_SMAGORINSKY);
+  default: OLB_BC_LAUNCH(K_BGK);
   }
 #undef OLB_BC_LAUNCH
-  return cudaGetLastError();
 }
 
 template <int Q, class S, class R>
@@ -177,27 +158,23 @@ cudaError_t launch_boundary(void* pops, const Geometry& g, bool shifted, const u
   cudaError_t e = cudaSuccess;
   if (n_flat) {
     const unsigned blocks = (n_flat + threads - 1) / threads;
-    bc_velocity_kernel<Q, S, R><<<blocks, threads, 0, stream>>>(static_cast<const S*>(pops), g, shifted, ids, t,
-                                                                cells, n_flat);
-    e = cudaGetLastError();
+    e = launch_chained(bc_velocity_kernel<Q, S, R>, true, blocks, threads, stream, static_cast<const S*>(pops), g,
+                       shifted, ids, t, cells, n_flat);
     if (e != cudaSuccess) return e;
-    plane_fd_kernel<Q, S, R><<<blocks, threads, 0, stream>>>(static_cast<S*>(pops), g, shifted, ids, t, periodic,
-                                                             cells, n_flat);
-    e = cudaGetLastError();
+    e = launch_chained(plane_fd_kernel<Q, S, R>, true, blocks, threads, stream, static_cast<S*>(pops), g, shifted, ids,
+                       t, periodic, cells, n_flat);
     if (e != cudaSuccess) return e;
   }
   if (n_edge) {
     const unsigned blocks = (n_edge + threads - 1) / threads;
-    outer_velocity_kernel<Q, S, R, false><<<blocks, threads, 0, stream>>>(
-      static_cast<S*>(pops), g, shifted, ids, t, periodic, cells + n_flat, n_edge);
-    e = cudaGetLastError();
+    e = launch_chained(outer_velocity_kernel<Q, S, R, false>, true, blocks, threads, stream, static_cast<S*>(pops), g,
+                       shifted, ids, t, periodic, cells + n_flat, n_edge);
     if (e != cudaSuccess) return e;
   }
   if (n_corner) {
     const unsigned blocks = (n_corner + threads - 1) / threads;
-    outer_velocity_kernel<Q, S, R, true><<<blocks, threads, 0, stream>>>(
-      static_cast<S*>(pops), g, shifted, ids, t, periodic, cells + n_flat + n_edge, n_corner);
-    e = cudaGetLastError();
+    e = launch_chained(outer_velocity_kernel<Q, S, R, true>, true, blocks, threads, stream, static_cast<S*>(pops), g,
+                       shifted, ids, t, periodic, cells + n_flat + n_edge, n_corner);
   }
   return e;
 }
@@ -216,7 +193,7 @@ cudaError_t launch_boundary(void* pops, const Geometry& g, bool shifted, const u
                                                const void*, void*, void*, cudaStream_t);           \
   template cudaError_t launch_boundary_collide<Q, S, R>(void*, const Geometry&, bool, const uint8_t*, \
                                                         const void*, int, const uint32_t*, uint32_t, \
-                                                        StatPartial*, cudaStream_t);               \
+                                                        const StatSink&, cudaStream_t);               \
   template cudaError_t launch_boundary<Q, S, R>(void*, const Geometry&, bool, const uint8_t*,      \
                                                 const void*, int, const uint32_t*, uint32_t,       \
                                                 uint32_t, uint32_t, cudaStream_t);                 \

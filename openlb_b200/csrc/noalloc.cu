@@ -59,17 +59,21 @@ using namespace olb_b200;
 
 namespace {
 
-// Scratch for the per-block statistics partials plus one slot for the reduced
-// result: (65536 + 1) * 40 B = 2.5 MiB per device.  A call with statistics
+// Scratch for the per-block statistics partials plus the reduced result:
+// 65536 * 40 B = 2.5 MiB per device.  A call with statistics
 // launches ceil(nz/bz) * ceil(ny/by) * nx blocks, (bz, by) = (128, 2) for
 // nz >= 128, (64, 4) for nz >= 64, else (32, 8): 65536 blocks cover a
 // 256 x 256 x 256 lattice, but only 2048 x 256 x 16 for a thin one.
 constexpr size_t kMaxBlocks = 65536;
-static __device__ __align__(256) StatPartial g_noalloc_scratch[kMaxBlocks + 1];
+struct Scratch {
+  StatPartial partials[kMaxBlocks];
+  StatResult result;
+};
+static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(Scratch)];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
-StatPartial* g_scratch_addr[kMaxDevices] = {};
+Scratch* g_scratch_addr[kMaxDevices] = {};
 
 olb_b200_status noalloc_fail(olb_b200_status code, const std::string& msg)
 {
@@ -86,14 +90,14 @@ olb_b200_status noalloc_cuda(cudaError_t e, const char* what)
 // looked up on the first call on that device and kept for the process: after
 // cudaDeviceReset on that device the kept address is stale, so callers that
 // reset a device must not use this entry point on it afterwards.
-olb_b200_status scratch_address(int device, StatPartial** out)
+olb_b200_status scratch_address(int device, Scratch** out)
 {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   if (!g_scratch_addr[device]) {
     void* ptr = nullptr;
     const cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
     if (e != cudaSuccess) return noalloc_cuda(e, "cudaGetSymbolAddress(scratch)");
-    g_scratch_addr[device] = static_cast<StatPartial*>(ptr);
+    g_scratch_addr[device] = static_cast<Scratch*>(ptr);
   }
   *out = g_scratch_addr[device];
   return OLB_B200_OK;
@@ -155,7 +159,7 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
 
   cudaError_t e = cudaSetDevice(desc->device);
   if (e != cudaSuccess) return noalloc_cuda(e, "cudaSetDevice");
-  StatPartial* scratch = nullptr;
+  Scratch* scratch = nullptr;
   olb_b200_status st = scratch_address(desc->device, &scratch);
   if (st != OLB_B200_OK) return st;
 
@@ -177,7 +181,8 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
     a.ids = nullptr;
     a.table = nullptr;
     a.bulk = params;
-    a.partials = last_stats ? scratch : nullptr;
+    if (last_stats) a.sink.partials = scratch->partials;
+    a.chained = k > 0;  // what the caller enqueued before is not overlapped
     a.block_z = bz;
     a.block_y = by;
     a.variant = variant;
@@ -205,12 +210,12 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   }
   if (!stats) return OLB_B200_OK;
 
-  StatPartial* result = scratch + kMaxBlocks;
-  reduce_partials_kernel<<<1, 1024, 0, s>>>(scratch, blocks, result);
-  e = cudaGetLastError();
+  // one block: no counter that calls overlapping by mistake could leave behind
+  e = launch_chained(reduce_partials_kernel, false, dim3(1), dim3(1024), s, scratch->partials, blocks, nullptr,
+                     &scratch->result, 0ull);
   if (e != cudaSuccess) return noalloc_cuda(e, "statistics reduction launch");
   StatPartial p;
-  e = cudaMemcpyAsync(&p, result, sizeof p, cudaMemcpyDeviceToHost, s);
+  e = cudaMemcpyAsync(&p, &scratch->result.p, sizeof p, cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return noalloc_cuda(e, "statistics read-back");
   e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return noalloc_cuda(e, "cudaStreamSynchronize");

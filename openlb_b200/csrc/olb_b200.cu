@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -35,7 +36,7 @@ namespace olb_b200 {
   extern template cudaError_t launch_boundary_collide<Q, S, R>(void*, const Geometry&, bool,       \
                                                                const uint8_t*, const void*, int,   \
                                                                const uint32_t*, uint32_t,          \
-                                                               StatPartial*, cudaStream_t);        \
+                                                               const StatSink&, cudaStream_t);        \
   extern template cudaError_t launch_boundary<Q, S, R>(void*, const Geometry&, bool, const uint8_t*, \
                                                        const void*, int, const uint32_t*, uint32_t, \
                                                        uint32_t, uint32_t, cudaStream_t);
@@ -48,31 +49,20 @@ OLB_B200_EXTERN(27, double, double)
 OLB_B200_EXTERN(27, __half, float)
 OLB_B200_EXTERN(27, __nv_bfloat16, float)
 
-__global__ void reduce_partials_kernel(const StatPartial* __restrict__ parts, size_t count,
-                                       StatPartial* __restrict__ out)
+__global__ void reduce_partials_kernel(const StatPartial* parts, size_t count, StatStage* stage, StatResult* out,
+                                       unsigned long long seq)
 {
-  // fixed assignment of partials to threads and a fixed tree: deterministic
-  double a = 0., b = 0., m = 0.;
-  unsigned long long n = 0, nf = 0;
-  for (size_t k = threadIdx.x; k < count; k += blockDim.x) {
-    const StatPartial p = parts[k];
-    a += p.sum_rho;
-    b += p.sum_usqr;
-    m = fmax(m, p.max_usqr);
-    n += p.n_cells;
-    nf += p.n_nonfinite;
+  next_may_start();
+  parts = after_previous(parts);
+  const size_t chunk = (count + gridDim.x - 1) / gridDim.x;
+  const size_t begin = blockIdx.x * chunk;
+  StatPartial sum = sum_partials(parts, begin < count ? begin : count, begin + chunk < count ? begin + chunk : count);
+  if (gridDim.x > 1) {
+    if (threadIdx.x == 0) stage->part[blockIdx.x] = sum;
+    if (!last_to_arrive(&stage->arrived, gridDim.x)) return;
+    sum = sum_partials(stage->part, 0, gridDim.x);
   }
-  __shared__ StatPartial sh[32];
-  warp_reduce(a, b, m, n, nf);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) sh[warp] = StatPartial{a, b, m, n, nf};
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    StatPartial p = lane < nw ? sh[lane] : StatPartial{0, 0, 0, 0, 0};
-    warp_reduce(p.sum_rho, p.sum_usqr, p.max_usqr, p.n_cells, p.n_nonfinite);
-    if (lane == 0) *out = p;
-  }
+  if (threadIdx.x == 0) write_result(out, sum, seq);
 }
 
 // velocity-change residual sums over the fluid cells; stores u as u_prev
@@ -80,7 +70,7 @@ template <class R>
 __global__ void velocity_residual_kernel(const R* __restrict__ u_now, R* __restrict__ u_prev,
                                          const uint8_t* __restrict__ ids,
                                          const DynDevice<R>* __restrict__ table, size_t cells,
-                                         StatPartial* __restrict__ partials)
+                                         const StatSink sink)
 {
   const size_t n = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
   double du2 = 0., u2 = 0.;
@@ -97,7 +87,7 @@ __global__ void velocity_residual_kernel(const R* __restrict__ u_now, R* __restr
       }
     }
   }
-  block_stats(du2, u2, 0., 0ull, 0ull, partials);
+  block_stats(du2, u2, 0., 0ull, 0ull, sink);
 }
 
 // splitmix64 (Steele, Lea, Flood, "Fast splittable pseudorandom number
@@ -117,10 +107,12 @@ OLB_HD uint64_t splitmix64(uint64_t x)
 template <class R>
 __global__ void bc_noise_kernel(const uint32_t* __restrict__ cells, uint32_t count,
                                 const uint8_t* __restrict__ ids, const DynDevice<R>* __restrict__ table,
-                                const R* __restrict__ base_all, R* __restrict__ values_all, Geometry g,
+                                const R* __restrict__ base_all, R* values_all, Geometry g,
                                 uint64_t step, uint64_t n_cells, double amp, uint64_t seed)
 {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  next_may_start();
+  values_all = after_previous(values_all);
   if (k >= count) return;
   const uint32_t n = cells[k];
   const DynDevice<R>* e = table + ids[n];
@@ -262,8 +254,9 @@ struct olb_b200_lattice {
   StatPartial* partials = nullptr;
   size_t n_partials = 0;
   void* uprev = nullptr;    // velocity at the last residual call (3 * cells * real)
-  StatPartial* stat_dev = nullptr;
-  StatPartial* stat_host = nullptr;  // pinned
+  StatStage* stat_stage = nullptr;
+  StatResult* stat_host = nullptr;   // pinned, written by the device
+  unsigned long long stat_seq = 0;   // number of the last reduction
   int block_z = 0, block_y = 0;
   int variant = 0;          // index of the step-kernel variant (step_variant)
   bool shape_fixed = false; // block_z, block_y (or flat tiles) chosen by the caller or the autotuner
@@ -461,6 +454,53 @@ olb_b200_status ensure_partials(olb_b200_lattice* L)
   return ensure_partial_count(L, step_blocks(L) + boundary_blocks(L));
 }
 
+// Blocks up to which the kernel that writes the partials also reduces them: its
+// last block then adds up at most four per thread, which is quicker than
+// another launch (32^3 cavity with statistics every step: 29.5 us a
+// step with reduction kernel, copy and synchronisation, 16.0 with this and
+// chained launches).  More go
+// through reduce_partials_kernel, one block per 1024.
+constexpr size_t kInKernelBlocks = 1024;
+
+// where a kernel of `blocks` blocks leaves its partials; in_kernel: no other
+// kernel adds to them
+StatSink stat_sink(olb_b200_lattice* L, size_t blocks, bool in_kernel)
+{
+  StatSink s;
+  s.partials = L->partials;
+  if (in_kernel && blocks <= kInKernelBlocks) {
+    s.stage = L->stat_stage;
+    s.result = L->stat_host;
+    s.seq = L->stat_seq + 1;
+  }
+  return s;
+}
+
+// Reduces `count` partials into stat_host unless their kernel did (reduced),
+// and waits for the result.  The device writes it into pinned memory with its
+// number last; the host polls for that number, which costs less than a copy
+// and a synchronisation, and looks at the stream's state now and then.
+olb_b200_status finish_stats(olb_b200_lattice* L, size_t count, bool reduced)
+{
+  const unsigned long long seq = ++L->stat_seq;
+  if (!reduced) {
+    const unsigned grid = unsigned(std::min<size_t>(kReduceBlocks, (count + 1023) / 1024));
+    const cudaError_t e = launch_chained(reduce_partials_kernel, true, dim3(grid), dim3(kReduceThreads), L->stream,
+                                         L->partials, count, L->stat_stage, L->stat_host, seq);
+    if (e != cudaSuccess) return cuda_fail(e, "statistics reduction launch");
+  }
+  const volatile unsigned long long* done = &L->stat_host->seq;
+  for (unsigned polls = 1; *done != seq; ++polls) {
+    if (polls % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(L->stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return cuda_fail(e, "statistics");
+    if (*done != seq) return fail(OLB_B200_ERR_CUDA, "statistics: the reduction left no result");
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return OLB_B200_OK;
+}
+
 olb_b200_status ensure_partial_count(olb_b200_lattice* L, size_t need)
 {
   if (need > L->n_partials) {
@@ -519,7 +559,8 @@ olb_b200_status enqueue_steps(olb_b200_lattice* L, int steps, bool stats_last)
     a.ids = L->masked ? L->ids : nullptr;
     a.table = L->table;
     a.bulk = L->bulk;
-    a.partials = stats ? L->partials : nullptr;
+    if (stats) a.sink = stat_sink(L, step_blocks(L), L->n_bc == 0);
+    a.chained = true;
     a.block_z = L->block_z;
     a.block_y = L->block_y;
     a.variant = L->variant;
@@ -528,7 +569,8 @@ olb_b200_status enqueue_steps(olb_b200_lattice* L, int steps, bool stats_last)
     cudaError_t e = cudaSuccess;
     if (L->n_bc) {
       // collision of the boundary cells in place, ahead of the step kernel
-      StatPartial* bp = stats ? L->partials + step_blocks(L) : nullptr;
+      StatSink bp;
+      if (stats) bp.partials = L->partials + step_blocks(L);
       e = dispatch(L, [&](auto qc, auto s_, auto r_) {
         return launch_boundary_collide<decltype(qc)::value, decltype(s_), decltype(r_)>(
           L->pops, L->g, odd, L->ids, L->table, L->bulk_kind, L->bc_cells, L->n_bc, bp, L->stream);
@@ -663,17 +705,16 @@ olb_b200_status boundary_noise(olb_b200_lattice* L)
   if (L->noise_amp == 0.0 || L->n_bc == 0) return OLB_B200_OK;
   const unsigned threads = 128, blocks = (L->n_bc + threads - 1) / threads;
   if (L->real == 8) {
-    bc_noise_kernel<double><<<blocks, threads, 0, L->stream>>>(
-      L->bc_cells, L->n_bc, L->ids, static_cast<const DynDevice<double>*>(L->table),
+    OLB_CUDA(launch_chained(
+      bc_noise_kernel<double>, true, dim3(blocks), dim3(threads), L->stream, L->bc_cells, L->n_bc, L->ids, static_cast<const DynDevice<double>*>(L->table),
       static_cast<const double*>(L->bc_base), static_cast<double*>(L->bc_values), L->g, uint64_t(L->steps_done),
-      uint64_t(L->cells), L->noise_amp, L->noise_seed);
+      uint64_t(L->cells), L->noise_amp, L->noise_seed));
   } else {
-    bc_noise_kernel<float><<<blocks, threads, 0, L->stream>>>(
-      L->bc_cells, L->n_bc, L->ids, static_cast<const DynDevice<float>*>(L->table),
+    OLB_CUDA(launch_chained(
+      bc_noise_kernel<float>, true, dim3(blocks), dim3(threads), L->stream, L->bc_cells, L->n_bc, L->ids, static_cast<const DynDevice<float>*>(L->table),
       static_cast<const float*>(L->bc_base), static_cast<float*>(L->bc_values), L->g, uint64_t(L->steps_done),
-      uint64_t(L->cells), L->noise_amp, L->noise_seed);
+      uint64_t(L->cells), L->noise_amp, L->noise_seed));
   }
-  OLB_CUDA(cudaGetLastError());
   return OLB_B200_OK;
 }
 
@@ -766,8 +807,10 @@ olb_b200_status olb_b200_create(const olb_b200_desc* desc, olb_b200_lattice** ou
   OLB_CUDA_C(cudaMemsetAsync(L->ids, 0, cells, L->stream));
   OLB_CUDA_C(cudaMalloc(&L->table, 256 * sizeof(DynDevice<double>)));
   OLB_CUDA_C(cudaMalloc(&L->scratch, 4 * cells * L->real));
-  OLB_CUDA_C(cudaMalloc(&L->stat_dev, sizeof(StatPartial)));
-  OLB_CUDA_C(cudaMallocHost(&L->stat_host, sizeof(StatPartial)));
+  OLB_CUDA_C(cudaMalloc(&L->stat_stage, sizeof(StatStage)));
+  OLB_CUDA_C(cudaMemsetAsync(L->stat_stage, 0, sizeof(StatStage), L->stream));
+  OLB_CUDA_C(cudaMallocHost(&L->stat_host, sizeof(StatResult)));
+  std::memset(L->stat_host, 0, sizeof(StatResult));
   L->device_bytes = pop_bytes + cells + 256 * sizeof(DynDevice<double>) + 4 * cells * L->real;
   // default: every cell NoDynamics
   olb_b200_dyn_params none{};
@@ -797,7 +840,7 @@ void olb_b200_destroy(olb_b200_lattice* L)
   if (L->bc_u) cudaFree(L->bc_u);
   if (L->bc_base) cudaFree(L->bc_base);
   if (L->force) cudaFree(L->force);
-  if (L->stat_dev) cudaFree(L->stat_dev);
+  if (L->stat_stage) cudaFree(L->stat_stage);
   if (L->stat_host) cudaFreeHost(L->stat_host);
   if (L->ev0) cudaEventDestroy(L->ev0);
   if (L->ev1) cudaEventDestroy(L->ev1);
@@ -1057,11 +1100,9 @@ olb_b200_status olb_b200_collide_and_stream(olb_b200_lattice* L, int32_t steps, 
   }
   if (!stats) return OLB_B200_OK;
   const size_t count = step_blocks(L) + boundary_blocks(L);
-  reduce_partials_kernel<<<1, 1024, 0, L->stream>>>(L->partials, count, L->stat_dev);
-  OLB_CUDA(cudaGetLastError());
-  OLB_CUDA(cudaMemcpyAsync(L->stat_host, L->stat_dev, sizeof(StatPartial), cudaMemcpyDeviceToHost, L->stream));
-  OLB_CUDA(cudaStreamSynchronize(L->stream));
-  const StatPartial p = *L->stat_host;
+  st = finish_stats(L, count, L->n_bc == 0 && count <= kInKernelBlocks);
+  if (st != OLB_B200_OK) return st;
+  const StatPartial p = L->stat_host->p;
   stats->sum_rho = p.sum_rho;
   stats->sum_usqr = p.sum_usqr;
   stats->max_usqr = p.max_usqr;
@@ -1203,21 +1244,20 @@ olb_b200_status olb_b200_velocity_residual(olb_b200_lattice* L, double* residual
   const size_t blocks = (L->cells + threads - 1) / threads;
   st = ensure_partial_count(L, blocks);
   if (st != OLB_B200_OK) return st;
+  const StatSink sink = stat_sink(L, blocks, true);
   if (L->real == 8) {
     velocity_residual_kernel<double><<<unsigned(blocks), threads, 0, L->stream>>>(
       reinterpret_cast<const double*>(u_d), static_cast<double*>(L->uprev), L->ids,
-      static_cast<const DynDevice<double>*>(L->table), L->cells, L->partials);
+      static_cast<const DynDevice<double>*>(L->table), L->cells, sink);
   } else {
     velocity_residual_kernel<float><<<unsigned(blocks), threads, 0, L->stream>>>(
       reinterpret_cast<const float*>(u_d), static_cast<float*>(L->uprev), L->ids,
-      static_cast<const DynDevice<float>*>(L->table), L->cells, L->partials);
+      static_cast<const DynDevice<float>*>(L->table), L->cells, sink);
   }
   OLB_CUDA(cudaGetLastError());
-  reduce_partials_kernel<<<1, 1024, 0, L->stream>>>(L->partials, blocks, L->stat_dev);
-  OLB_CUDA(cudaGetLastError());
-  OLB_CUDA(cudaMemcpyAsync(L->stat_host, L->stat_dev, sizeof(StatPartial), cudaMemcpyDeviceToHost, L->stream));
-  OLB_CUDA(cudaStreamSynchronize(L->stream));
-  const StatPartial p = *L->stat_host;
+  st = finish_stats(L, blocks, blocks <= kInKernelBlocks);
+  if (st != OLB_B200_OK) return st;
+  const StatPartial p = L->stat_host->p;
   *residual = p.sum_usqr > 0. ? std::sqrt(p.sum_rho / p.sum_usqr) : (p.sum_rho > 0. ? INFINITY : 0.);
   return OLB_B200_OK;
 }
