@@ -128,13 +128,20 @@ OLB_DEV int cell_kind(const float* __restrict__ pool, const InstanceDevice& I, u
   return CELL_FLUID;
 }
 
+// One step of every active instance.  Bounded by HBM: 152 B per cell and the
+// class byte.  Launched chained.  The class decides before the populations are
+// loaded: loading them with it, and dropping a wall cell's, took 305 us against
+// 276 for an odd step of 30 cavities with 9.3 M cells (269 against 269 for an
+// even one); so did every form that spilled under the 64-register cap.
 template <int MINB>
 __global__ void __launch_bounds__(kEnsembleThreads, MINB)
 ensemble_step_kernel(float* __restrict__ pool, const InstanceDevice* __restrict__ table,
                      const Tile* __restrict__ tiles, const int* __restrict__ ntiles_ptr, int k_in_chunk)
 {
   using L = L19;
+  next_may_start();
   const int ntiles = *ntiles_ptr;
+  after_previous(pool);  // (through the returned pointer the kernel spills; pool's loads are ordinary ones)
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const Tile tile = tiles[t];
     const InstanceDevice& I = table[tile.inst];
@@ -225,91 +232,113 @@ ensemble_step_kernel(float* __restrict__ pool, const InstanceDevice* __restrict_
 // logical post-stream state of every fluid cell against the stored one (then
 // stored), summed per tile in FP64 with a fixed-order block reduction.  The
 // same quantity as olb_b200_velocity_residual on a single lattice.
+// One block per tile, as the step kernel: a fixed grid of a few blocks per SM
+// that walked the tiles had two barriers and a chain of dependent loads per
+// tile in its way (1481 us for 9.3 M cells, 169 us with a block per tile).
 __global__ void __launch_bounds__(kEnsembleThreads)
 ensemble_check_kernel(float* __restrict__ pool, const InstanceDevice* __restrict__ table,
                       const Tile* __restrict__ tiles, const int* __restrict__ ntiles_ptr, int steps_in_chunk,
                       ResidualPartial* __restrict__ partials)
 {
   using L = L19;
-  const int ntiles = *ntiles_ptr;
+  const int t = blockIdx.x;
+  if (t >= *ntiles_ptr) return;
   __shared__ double sh[2][kEnsembleThreads / 32];
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile tile = tiles[t];
-    const InstanceDevice& I = table[tile.inst];
-    double du2 = 0., u2 = 0.;
-    if (I.active) {
-      const bool shifted = ((I.steps_done + uint32_t(steps_in_chunk)) & 1u) != 0u;
-      const float* __restrict__ pops = pool + I.pops;
-      float* __restrict__ up = pool + I.uprev;
-      const Geometry g{I.nx, I.ny, I.nz, I.stride, 0};
-      for (int k = 0; k < kTileCells; ++k) {
-        const uint32_t n = tile.start + threadIdx.x + uint32_t(k) * kEnsembleThreads;
-        if (n >= I.cells) break;
-        const uint32_t x = I.div_nynz.div(n);
-        const uint32_t r = n - x * I.nynz;
-        const uint32_t y = I.div_nz.div(r);
-        const uint32_t z = r - y * I.nz_u;
-        if (cell_kind(pool, I, n, int(x), int(y), int(z)) != CELL_FLUID) continue;
-        float f[kQ];
-        static_for<0, kQ>([&](auto i) {
-          f[i] = logical_pop<kQ, float, float, i.value>(pops, g, int(x), int(y), int(z), shifted);
-        });
-        float rho, u[3];
-        if (I.forced) {
-          const float gg[3] = {I.force[0], I.force[1], I.force[2]};
-          compute_rho_u_forced<L>(f, gg, rho, u);
-        } else {
-          compute_rho_u<L>(f, rho, u);
-        }
-        for (int d = 0; d < 3; ++d) {
-          const double du = double(u[d]) - double(up[size_t(d) * I.stride + n]);
-          du2 += du * du;
-          u2 += double(u[d]) * double(u[d]);
-          up[size_t(d) * I.stride + n] = u[d];
-        }
+  const Tile tile = tiles[t];
+  const InstanceDevice& I = table[tile.inst];
+  double du2 = 0., u2 = 0.;
+  const uint32_t n = tile.start + threadIdx.x;
+  if (I.active && n < I.cells) {
+    const bool shifted = ((I.steps_done + uint32_t(steps_in_chunk)) & 1u) != 0u;
+    const float* __restrict__ pops = pool + I.pops;
+    float* __restrict__ up = pool + I.uprev;
+    const Geometry g{I.nx, I.ny, I.nz, I.stride, 0};
+    const uint32_t x = I.div_nynz.div(n);
+    const uint32_t r = n - x * I.nynz;
+    const uint32_t y = I.div_nz.div(r);
+    const uint32_t z = r - y * I.nz_u;
+    if (cell_kind(pool, I, n, int(x), int(y), int(z)) == CELL_FLUID) {
+      float before[3];
+      for (int d = 0; d < 3; ++d) before[d] = up[size_t(d) * I.stride + n];
+      float f[kQ];
+      load_logical<kQ, float, float>(pops, g, int(x), int(y), int(z), shifted, f);
+      float rho, u[3];
+      if (I.forced) {
+        const float gg[3] = {I.force[0], I.force[1], I.force[2]};
+        compute_rho_u_forced<L>(f, gg, rho, u);
+      } else {
+        compute_rho_u<L>(f, rho, u);
+      }
+      for (int d = 0; d < 3; ++d) {
+        const double du = double(u[d]) - double(before[d]);
+        du2 += du * du;
+        u2 += double(u[d]) * double(u[d]);
+        up[size_t(d) * I.stride + n] = u[d];
       }
     }
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      du2 += __shfl_down_sync(0xffffffffu, du2, o);
-      u2 += __shfl_down_sync(0xffffffffu, u2, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    du2 += __shfl_down_sync(0xffffffffu, du2, o);
+    u2 += __shfl_down_sync(0xffffffffu, u2, o);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) {
+    sh[0][warp] = du2;
+    sh[1][warp] = u2;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double a = 0., b = 0.;
+    for (int w = 0; w < kEnsembleThreads / 32; ++w) {
+      a += sh[0][w];
+      b += sh[1][w];
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-      sh[0][warp] = du2;
-      sh[1][warp] = u2;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double a = 0., b = 0.;
-      for (int w = 0; w < kEnsembleThreads / 32; ++w) {
-        a += sh[0][w];
-        b += sh[1][w];
-      }
-      partials[t] = ResidualPartial{a, b};
-    }
-    __syncthreads();
+    partials[t] = ResidualPartial{a, b};
   }
 }
 
-// per instance: reduce its contiguous tile range in order; advance steps_done
-__global__ void ensemble_finish_kernel(InstanceDevice* __restrict__ table, const int* __restrict__ tile_begin,
-                                       const int* __restrict__ tile_end, const int* __restrict__ ninst_ptr,
-                                       int steps, int check, const ResidualPartial* __restrict__ partials,
-                                       double* __restrict__ residual_out, uint32_t* __restrict__ steps_out)
+// One block per slot: reduces the instance's contiguous tile range (a fixed
+// assignment of its tiles to threads and a fixed tree, so the sum does not
+// depend on the mix) and advances steps_done.  One thread per instance, adding
+// its tiles one after the other, took 461 us for the largest of 30 (93^3 cells,
+// 3143 tiles); this takes 9 us.
+constexpr int kFinishThreads = 128;
+__global__ void __launch_bounds__(kFinishThreads)
+ensemble_finish_kernel(InstanceDevice* __restrict__ table, const int* __restrict__ tile_begin,
+                       const int* __restrict__ tile_end, int steps, int check,
+                       const ResidualPartial* __restrict__ partials, double* __restrict__ residual_out,
+                       uint32_t* __restrict__ steps_out)
 {
-  const int ninst = *ninst_ptr;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ninst) return;
+  const int s = blockIdx.x;
   InstanceDevice& I = table[s];
   if (!I.active) return;
-  I.steps_done += uint32_t(steps);
-  steps_out[s] = I.steps_done;
-  if (check) {
-    double a = 0., b = 0.;
-    for (int t = tile_begin[s]; t < tile_end[s]; ++t) {
-      a += partials[t].du2;
-      b += partials[t].u2;
+  if (threadIdx.x == 0) {
+    I.steps_done += uint32_t(steps);
+    steps_out[s] = I.steps_done;
+  }
+  if (!check) return;
+  double a = 0., b = 0.;
+  for (int t = tile_begin[s] + int(threadIdx.x); t < tile_end[s]; t += kFinishThreads) {
+    a += partials[t].du2;
+    b += partials[t].u2;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  __shared__ double sh[2][kFinishThreads / 32];
+  if ((threadIdx.x & 31) == 0) {
+    sh[0][threadIdx.x >> 5] = a;
+    sh[1][threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a = b = 0.;
+    for (int w = 0; w < kFinishThreads / 32; ++w) {
+      a += sh[0][w];
+      b += sh[1][w];
     }
     residual_out[s] = b > 0. ? sqrt(a / b) : (a > 0. ? INFINITY : 0.);
   }
@@ -335,9 +364,7 @@ __global__ void ensemble_moments_kernel(const float* __restrict__ pool, Instance
     const Geometry g{I.nx, I.ny, I.nz, I.stride, 0};
     const float* pops = pool + I.pops;
     float f[kQ];
-    static_for<0, kQ>([&](auto i) {
-      f[i] = logical_pop<kQ, float, float, i.value>(pops, g, int(x), int(y), int(z), shifted);
-    });
+    load_logical<kQ, float, float>(pops, g, int(x), int(y), int(z), shifted, f);
     if (I.forced) {
       const float gg[3] = {I.force[0], I.force[1], I.force[2]};
       compute_rho_u_forced<L>(f, gg, rho, u);
@@ -381,8 +408,7 @@ struct olb_b200_ensemble {
   float* moments_dev = nullptr;                // staging for get_moments
   size_t moments_cap = 0;
   bool dirty = true;                           // tables changed since upload
-  int grid = 0;                                // persistent grid of the check kernel
-  int step_grid = 0;                           // blocks of the step kernel: ntiles rounded up
+  int step_grid = 0;                           // blocks of the step and check kernels: ntiles rounded up
   int min_blocks = 4;
   cudaStream_t stream = nullptr;
   cudaGraphExec_t graph = nullptr;
@@ -515,32 +541,19 @@ olb_b200_status upload_tables(olb_b200_ensemble* E)
 olb_b200_status enqueue_chunk(olb_b200_ensemble* E, int steps, int check)
 {
   for (int k = 0; k < steps; ++k) {
-    switch (E->min_blocks) {
-    case 2:
-      ensemble_step_kernel<2><<<E->step_grid, kEnsembleThreads, 0, E->stream>>>(
-        E->pool, E->table_dev, E->tiles_dev, E->counts_dev, k);
-      break;
-    case 4:
-      ensemble_step_kernel<4><<<E->step_grid, kEnsembleThreads, 0, E->stream>>>(
-        E->pool, E->table_dev, E->tiles_dev, E->counts_dev, k);
-      break;
-    default:
-      ensemble_step_kernel<3><<<E->step_grid, kEnsembleThreads, 0, E->stream>>>(
-        E->pool, E->table_dev, E->tiles_dev, E->counts_dev, k);
-      break;
-    }
-    OLB_ECUDA(cudaGetLastError());
+    const auto kernel = E->min_blocks == 2   ? ensemble_step_kernel<2>
+                        : E->min_blocks == 4 ? ensemble_step_kernel<4>
+                                             : ensemble_step_kernel<3>;
+    OLB_ECUDA(launch_chained(kernel, k > 0, dim3(unsigned(E->step_grid)), dim3(kEnsembleThreads), E->stream, E->pool,
+                             E->table_dev, E->tiles_dev, E->counts_dev, k));
   }
   if (check) {
-    ensemble_check_kernel<<<E->grid, kEnsembleThreads, 0, E->stream>>>(E->pool, E->table_dev, E->tiles_dev,
+    ensemble_check_kernel<<<E->step_grid, kEnsembleThreads, 0, E->stream>>>(E->pool, E->table_dev, E->tiles_dev,
                                                                        E->counts_dev, steps, E->partials);
     OLB_ECUDA(cudaGetLastError());
   }
-  const int threads = 128;
-  const int blocks = (E->max_instances + threads - 1) / threads;
-  ensemble_finish_kernel<<<blocks, threads, 0, E->stream>>>(E->table_dev, E->tile_begin_dev, E->tile_end_dev,
-                                                             E->counts_dev + 1, steps, check, E->partials,
-                                                             E->residual_dev, E->steps_dev);
+  ensemble_finish_kernel<<<E->max_instances, kFinishThreads, 0, E->stream>>>(
+    E->table_dev, E->tile_begin_dev, E->tile_end_dev, steps, check, E->partials, E->residual_dev, E->steps_dev);
   OLB_ECUDA(cudaGetLastError());
   OLB_ECUDA(cudaMemcpyAsync(E->residual_host, E->residual_dev, size_t(E->max_instances) * sizeof(double),
                             cudaMemcpyDeviceToHost, E->stream));
@@ -593,10 +606,7 @@ olb_b200_status olb_b200_ensemble_create(const olb_b200_ensemble_desc* desc, olb
   OLB_ECUDA_C(cudaMallocHost(&E->steps_host, size_t(E->max_instances) * sizeof(uint32_t)));
   OLB_ECUDA_C(cudaMemsetAsync(E->residual_dev, 0, size_t(E->max_instances) * sizeof(double), E->stream));
   OLB_ECUDA_C(cudaMemsetAsync(E->steps_dev, 0, size_t(E->max_instances) * sizeof(uint32_t), E->stream));
-  int sms = 0;
-  OLB_ECUDA_C(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
   E->min_blocks = 4;
-  E->grid = sms * E->min_blocks;
   olb_b200_status st = upload_tables(E);
   if (st != OLB_B200_OK) return cleanup(st);
 #undef OLB_ECUDA_C
@@ -825,10 +835,7 @@ olb_b200_status olb_b200_ensemble_set_occupancy(olb_b200_ensemble* E, int32_t bl
   detail::set_last_error("");
   if (!E || (blocks_per_sm != 2 && blocks_per_sm != 3 && blocks_per_sm != 4))
     return efail(OLB_B200_ERR_ARG, "ensemble_set_occupancy: blocks_per_sm must be 2, 3 or 4");
-  int sms = 0;
-  OLB_ECUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
   E->min_blocks = blocks_per_sm;
-  E->grid = sms * blocks_per_sm;
   if (E->graph) {
     cudaGraphExecDestroy(E->graph);
     E->graph = nullptr;
