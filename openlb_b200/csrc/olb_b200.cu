@@ -18,6 +18,7 @@
 
 #include "../../include/olb_b200.h"
 #include "aa_kernels.cuh"
+#include "step_defaults.cuh"
 
 namespace olb_b200 {
 
@@ -307,20 +308,7 @@ void default_shape(const olb_b200_lattice* L, int& bz, int& by)
   by = 256 / bz;
 }
 
-// Default step variant per lattice class, from a 256^3 sweep on B200 (the
-// autotuner refines it on the actual lattice): masked lattices and 16-bit
-// storage keep one cell per thread at high occupancy; FP64 and unmasked
-// FP32 lattices issue the loads of two cells per thread.
-int default_variant(const olb_b200_lattice* L)
-{
-  const int storage = L->desc.storage;
-  // 16-bit: D3Q19's two-lane collision fits the 64-register cap of {1,4};
-  // D3Q27's needs the 80 registers of {1,3}
-  if (storage == OLB_B200_STORAGE_F16 || storage == OLB_B200_STORAGE_BF16) return L->q == 27 ? 0 : 1;
-  if (L->masked) return storage == OLB_B200_STORAGE_F64 ? 0 : 1;                  // {1,3} / {1,4}
-  if (storage == OLB_B200_STORAGE_F64) return 2;                                     // {2,2}
-  return 3;                                                                          // {2,3}
-}
+int default_variant(const olb_b200_lattice* L) { return default_step_variant(L->q, int(L->elem), L->masked); }
 
 int cells_per_thread(const olb_b200_lattice* L)
 {
