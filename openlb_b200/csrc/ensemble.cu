@@ -34,6 +34,7 @@
 
 #include "../../include/olb_b200.h"
 #include "aa_kernels.cuh"
+#include "host_copy.h"
 
 namespace olb_b200 {
 namespace detail {
@@ -386,6 +387,7 @@ struct Region {
 } // namespace
 
 struct olb_b200_ensemble {
+  HostCopyHold host_copy;
   int device = 0;
   int max_instances = 0;
   uint64_t pool_elems = 0;
@@ -804,9 +806,8 @@ olb_b200_status olb_b200_ensemble_get_moments(olb_b200_ensemble* E, int32_t slot
   float* dev = E->moments_dev;
   ensemble_moments_kernel<<<(I.cells + 255) / 256, 256, 0, E->stream>>>(E->pool, I, dev, dev + I.cells);
   OLB_ECUDA(cudaGetLastError());
-  OLB_ECUDA(cudaMemcpyAsync(host_rho, dev, size_t(I.cells) * sizeof(float), cudaMemcpyDeviceToHost, E->stream));
-  OLB_ECUDA(cudaMemcpyAsync(host_u, dev + I.cells, size_t(I.cells) * 3 * sizeof(float), cudaMemcpyDeviceToHost,
-                            E->stream));
+  OLB_ECUDA(copy_to_host(host_rho, dev, size_t(I.cells) * sizeof(float), E->device, E->stream));
+  OLB_ECUDA(copy_to_host(host_u, dev + I.cells, size_t(I.cells) * 3 * sizeof(float), E->device, E->stream));
   OLB_ECUDA(cudaStreamSynchronize(E->stream));
   return OLB_B200_OK;
 }

@@ -151,8 +151,9 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
     return noalloc_fail(OLB_B200_ERR_ARG, buf);
   }
   // The step kernel a handle's unmasked lattice takes (a 256^3 FP32 box: 394 us
-  // per step with two cells per thread, 432 with one).  Flat tiles of kStepThreads, which a step with
-  // statistics takes, need no more blocks than the limit counts.
+  // per step with two cells per thread, 432 with one).  Flat tiles of
+  // kStepThreads, which a step with statistics takes, need no more blocks than
+  // the limit counts.
   const int variant = default_step_variant(desc->q, elem, false);
   set_flat(g, kStepThreads);
   const dim3 stat_grid = step_grid(g, bz, by, step_cells(g, elem, variant));

@@ -18,6 +18,7 @@
 
 #include "../../include/olb_b200.h"
 #include "aa_kernels.cuh"
+#include "host_copy.h"
 #include "step_defaults.cuh"
 
 namespace olb_b200 {
@@ -234,6 +235,7 @@ void set_last_error(const std::string& message) { g_last_error = message; }
 } // namespace olb_b200
 
 struct olb_b200_lattice {
+  HostCopyHold host_copy;
   olb_b200_desc desc{};
   int q = 19;
   size_t cells = 0;
@@ -1037,9 +1039,8 @@ olb_b200_status olb_b200_get_populations(olb_b200_lattice* L, void* host_pops)
   char* dst = static_cast<char*>(host_pops);
   if (L->elem == L->real && L->parity == 0) {
     for (int i = 0; i < L->q; ++i) {
-      OLB_CUDA(cudaMemcpyAsync(dst + size_t(i) * col,
-                               static_cast<const char*>(L->pops) + size_t(i) * L->stride * L->elem, col,
-                               cudaMemcpyDeviceToHost, L->stream));
+      OLB_CUDA(copy_to_host(dst + size_t(i) * col, static_cast<const char*>(L->pops) + size_t(i) * L->stride * L->elem,
+                            col, L->device, L->stream));
     }
   } else {
     for (int i0 = 0; i0 < L->q; i0 += 4) {
@@ -1049,8 +1050,7 @@ olb_b200_status olb_b200_get_populations(olb_b200_lattice* L, void* host_pops)
                                                                              L->scratch, i0, i1, L->stream);
       });
       if (e != cudaSuccess) return cuda_fail(e, "gather kernel");
-      OLB_CUDA(cudaMemcpyAsync(dst + size_t(i0) * col, L->scratch, size_t(i1 - i0) * col,
-                               cudaMemcpyDeviceToHost, L->stream));
+      OLB_CUDA(copy_to_host(dst + size_t(i0) * col, L->scratch, size_t(i1 - i0) * col, L->device, L->stream));
     }
   }
   OLB_CUDA(cudaStreamSynchronize(L->stream));
@@ -1121,8 +1121,8 @@ olb_b200_status olb_b200_get_moments(olb_b200_lattice* L, void* host_rho, void* 
       L->pops, L->g, L->parity == 1, L->ids, L->table, rho_d, u_d, L->stream);
   });
   if (e != cudaSuccess) return cuda_fail(e, "moments kernel");
-  OLB_CUDA(cudaMemcpyAsync(host_rho, rho_d, L->cells * L->real, cudaMemcpyDeviceToHost, L->stream));
-  OLB_CUDA(cudaMemcpyAsync(host_u, u_d, 3 * L->cells * L->real, cudaMemcpyDeviceToHost, L->stream));
+  OLB_CUDA(copy_to_host(host_rho, rho_d, L->cells * L->real, L->device, L->stream));
+  OLB_CUDA(copy_to_host(host_u, u_d, 3 * L->cells * L->real, L->device, L->stream));
   OLB_CUDA(cudaStreamSynchronize(L->stream));
   return OLB_B200_OK;
 }
