@@ -310,7 +310,10 @@ void default_shape(const olb_b200_lattice* L, int& bz, int& by)
   by = 256 / bz;
 }
 
-int default_variant(const olb_b200_lattice* L) { return default_step_variant(L->q, int(L->elem), L->masked); }
+int default_variant(const olb_b200_lattice* L)
+{
+  return default_step_variant(L->q, int(L->elem), L->masked, L->bulk_kind, L->cells);
+}
 
 int cells_per_thread(const olb_b200_lattice* L)
 {

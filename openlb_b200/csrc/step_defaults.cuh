@@ -1,19 +1,38 @@
 // Which step kernel a lattice takes unless told otherwise.
 #pragma once
 
+#include <cstddef>
+
+#include "aa_kernels.cuh"
+
 namespace olb_b200 {
 
-// Default step variant per lattice class, from a 256^3 sweep on B200 (the
-// autotuner refines it on the actual lattice): masked lattices and 16-bit
-// storage keep one cell per thread at high occupancy; FP64 and unmasked
-// FP32 lattices issue the loads of two cells per thread.
-inline int default_step_variant(int q, int bytes, bool masked)
+// Default step variant per lattice class (the autotuner refines it on the
+// actual lattice), from sweeps of cubes of 16..320 cells a side on B200, chained
+// launches, us per step:
+//   A lattice whose threads all fit the SMs at 3 blocks of 256 takes {1,3}: a
+// fourth block per SM has nothing to run and costs registers.  Masked 48^3 (one
+// wave) {1,3} 3.71 against {1,4} 4.25 in FP32, 3.84 against 5.77 in FP16 forced
+// TRT; 52^3 (two waves) 4.83 against 4.15.  16-bit kernels hold two cells per
+// thread: FP16 60^3 3.80 against 4.36, 64^3 4.43 against 4.23.
+//   16-bit: D3Q19's two-lane collision fits the 64 registers of {1,4}; D3Q27's
+// needs the 80 of {1,3} (160^3 masked BF16 81.6 against 92.9).
+//   FP64: {1,3} (160^3 D3Q19 masked 189 against 191 {1,4}; D3Q27 128^3 140 against
+// 164 {1,4} and 146 {2,2}).
+//   FP32: {1,4} (64^3 open 5.80 against 6.49 {2,3}, 256^3 open forced TRT 417
+// against 430), but two cells per thread {2,3} where they win: from 2^21 cells
+// open boxes without a force (256^3 389 against 393, 160^3 100.0 against 99.4 but
+// 3 % less with statistics every step, 96^3 16.2 against 15.9) and masked
+// lattices with one (200^3 207 against 214, 128^3 57.4 against 58.4, 96^3 20.2
+// against 19.6).
+inline int default_step_variant(int q, int bytes, bool masked, int kind, size_t cells)
 {
-  // 16-bit: D3Q19's two-lane collision fits the 64-register cap of {1,4};
-  // D3Q27's needs the 80 registers of {1,3}
+  constexpr size_t kOneWave = size_t(148) * 3 * kStepThreads;
+  const bool one_wave = (bytes == 2 ? (cells + 1) / 2 : cells) <= kOneWave;
+  if (bytes == 8 || one_wave) return 0;
   if (bytes == 2) return q == 27 ? 0 : 1;
-  if (masked) return bytes == 8 ? 0 : 1;  // {1,3} / {1,4}
-  return bytes == 8 ? 2 : 3;              // {2,2} / {2,3}
+  const bool forced = kind == K_FORCED_BGK || kind == K_FORCED_TRT;
+  return forced == masked && cells >= size_t(1) << 21 ? 3 : 1;
 }
 
 } // namespace olb_b200
