@@ -21,7 +21,9 @@
  *     the last stream.  The element type is the compute type: double for
  *     OLB_B200_STORAGE_F64, float otherwise.  How the library keeps them in
  *     device memory (AA pattern, 16-bit storage) is internal.
- *   - Host pointers are borrowed for the duration of the call.  Device
+ *   - Host pointers are borrowed for the duration of the call.  Results copied
+ *     into memory that is not pinned pass through pinned buffers that all
+ *     handles of a process share (8 MiB, given back with the last handle).  Device
  *     memory, the CUDA stream and any CUDA graphs are owned by the handle.
  *   - One host thread drives one lattice handle; distinct handles may be used
  *     from distinct threads.  All device work of a handle is ordered on its
@@ -272,7 +274,10 @@ olb_b200_status olb_b200_get_info(olb_b200_lattice* lattice, int64_t* steps_done
                                   int64_t* device_bytes, int32_t* block_z, int32_t* block_y);
 
 /* Launch shape of the step kernel (threads along z and y, product <= 256,
- * block_z a multiple of 32).  0,0 selects the built-in default. */
+ * block_z a multiple of 32).  0,0 selects the built-in default: blocks of
+ * consecutive cells of a plane's y-z index, which leave no lane without a cell
+ * whatever the extents (olb_b200_get_info then reports the nearest rectangle).
+ * 16-bit lattices with odd nx always run the default. */
 olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* lattice, int32_t block_z, int32_t block_y);
 
 /* Step-kernel tuning.  The library compiles a few variants of the step kernel
@@ -289,8 +294,8 @@ typedef struct {
   float ms_per_step;          /* best time per step measured by autotune, else 0 */
 } olb_b200_tuning;
 
-/* Times every (variant, launch shape) pair on this lattice for trial_steps
- * steps each (0: 4) and keeps the fastest.  The lattice state is copied to a
+/* Times every (variant, launch shape) pair, the built-in default among the
+ * shapes, on this lattice for trial_steps steps each (0: 4) and keeps the fastest.  The lattice state is copied to a
  * temporary device buffer first and restored afterwards, so the simulation does
  * not advance.  Synchronous. */
 olb_b200_status olb_b200_autotune(olb_b200_lattice* lattice, int32_t trial_steps, olb_b200_tuning* out);

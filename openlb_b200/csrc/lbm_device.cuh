@@ -1134,9 +1134,12 @@ OLB_DEV void relax_scaled(V (&g)[L::q], const V (&ps)[L::half + 1], const V (&pd
     if constexpr (FORCED) {
       const V kf = v_mul(v_splat<V>(T), fr);
       a0 = v_fma(v_mul(v_splat<V>(-1.f), kf), uf3, a0);
-      const V cf = rep_dot<L, p.value>(gf);
-      A = v_fma(v_mul(wt, rho45), v_mul(cu, cu), v_fma(v_mul(v_splat<V>(9.f), kf), v_mul(cu, cf), a0));
-      B = v_fma(v_mul(v_splat<V>(K), rho_odd), cu, v_mul(v_mul(v_splat<V>(3.f), kf), cf));
+      // fb = 3 kf (c.F) serves both parts: A = a0 + (c.u) (wt rho45 (c.u) + 3 fb)
+      // takes one operation less than its two products with (c.u) apart
+      // (256^3 FP16 forced TRT 230.5 -> 222.8 us, porous 384x192x192 219.7 -> 215.2)
+      const V fb = v_mul(v_mul(v_splat<V>(3.f), kf), rep_dot<L, p.value>(gf));
+      A = v_fma(v_fma(v_splat<V>(3.f), fb, v_mul(v_mul(wt, rho45), cu)), cu, a0);
+      B = v_fma(v_mul(v_splat<V>(K), rho_odd), cu, fb);
     } else {
       A = v_fma(v_mul(wt, rho45), v_mul(cu, cu), a0);
       B = v_mul(v_mul(v_splat<V>(K), rho_odd), cu);
@@ -1148,14 +1151,25 @@ OLB_DEV void relax_scaled(V (&g)[L::q], const V (&ps)[L::half + 1], const V (&pd
   });
 }
 
+// the first pair of weight class k with c_a c_b != 0, 0 when there is none
+template <class L>
+OLB_HD constexpr int first_pair_on_axes(int a, int b, int k)
+{
+  for (int p = 1; p <= L::half; ++p) {
+    if (weight_class<L>(p) == k && L::c(pair_rep<L>(p), a) * L::c(pair_rep<L>(p), b) != 0) return p;
+  }
+  return 0;
+}
+
 // Smagorinsky effective omega from the scaled populations: Pi_ab per weight
-// class from the pair sums, one multiply by 1/s per class.
+// class from the pair sums, one multiply by 1/s per class.  Sums start from
+// their first term (an addition to zero is not folded away; the results are the
+// same), and a class without a term costs nothing.
 template <class L, class V>
 OLB_DEV V smagorinsky_omega_scaled(const V (&ps)[L::half + 1], const V& rho, const V& rinv, const V& delta,
                                    const V (&u)[3], const V& smago_pre, const V& tau_mol)
 {
   V pik[6][4];
-  static_for<0, 6>([&](auto m) { static_for<0, 4>([&](auto k) { pik[m][k] = v_splat<V>(-0.f); }); });
   static_for<1, L::half + 1>([&](auto p) {
     constexpr int k = weight_class<L>(p.value);
     constexpr int r = pair_rep<L>(p.value);
@@ -1163,7 +1177,10 @@ OLB_DEV V smagorinsky_omega_scaled(const V (&ps)[L::half + 1], const V& rho, con
       static_for<a.value, 3>([&](auto b) {
         constexpr int m = a.value * 3 - (a.value * (a.value - 1)) / 2 + (b.value - a.value);
         constexpr int cc = L::c(r, a) * L::c(r, b);
-        if constexpr (cc == 1) { pik[m][k] = v_add(pik[m][k], ps[p]); }
+        constexpr bool first = first_pair_on_axes<L>(a, b, k) == p.value;
+        if constexpr (first && cc == 1) { pik[m][k] = ps[p]; }
+        else if constexpr (first && cc == -1) { pik[m][k] = v_mul(ps[p], v_splat<V>(-1.f)); }
+        else if constexpr (cc == 1) { pik[m][k] = v_add(pik[m][k], ps[p]); }
         else if constexpr (cc == -1) { pik[m][k] = v_sub(pik[m][k], ps[p]); }
       });
     });
@@ -1172,10 +1189,14 @@ OLB_DEV V smagorinsky_omega_scaled(const V (&ps)[L::half + 1], const V& rho, con
   static_for<0, 3>([&](auto a) {
     static_for<a.value, 3>([&](auto b) {
       constexpr int m = a.value * 3 - (a.value * (a.value - 1)) / 2 + (b.value - a.value);
-      V s = v_splat<V>(-0.f);
+      V s;
       static_for<1, 4>([&](auto k) {
+        constexpr bool any = first_pair_on_axes<L>(a, b, k) != 0;
+        constexpr bool first = any && (k == 1 || first_pair_on_axes<L>(a, b, 1) == 0) &&
+                               (k <= 2 || first_pair_on_axes<L>(a, b, 2) == 0);
         constexpr float inv = inv_class_scale<L>(k);
-        if constexpr (inv != 0.f) { s = v_fma(pik[m][k], v_splat<V>(inv), s); }
+        if constexpr (first) { s = v_mul(pik[m][k], v_splat<V>(inv)); }
+        else if constexpr (any) { s = v_fma(pik[m][k], v_splat<V>(inv), s); }
       });
       s = v_sub(s, v_mul(v_mul(rho, u[a]), u[b]));
       if constexpr (a.value == b.value) { s = v_sub(s, v_mul(v_splat<V>(1.f / 3.f), delta)); }
