@@ -118,7 +118,17 @@ cudaError_t launch_moments(const void* pops, const Geometry& g, bool shifted, co
                            const void* table, void* rho, void* u, cudaStream_t stream)
 {
   const dim3 block(32, 8);
-  const dim3 grid = cell_grid(g, 32, 8);
+  dim3 grid = cell_grid(g, 32, 8);
+  constexpr bool kHalf = std::is_same_v<S, __half> || std::is_same_v<S, __nv_bfloat16>;
+  if constexpr (kHalf) {
+    if (g.paired) {
+      grid.z /= 2;
+      moments_paired_kernel<Q, S><<<grid, block, 0, stream>>>(
+        static_cast<const S*>(pops), g, shifted, ids, static_cast<const DynDevice<float>*>(table),
+        static_cast<float*>(rho), static_cast<float*>(u));
+      return cudaGetLastError();
+    }
+  }
   moments_kernel<Q, S, R><<<grid, block, 0, stream>>>(static_cast<const S*>(pops), g, shifted, ids,
                                                        static_cast<const DynDevice<R>*>(table),
                                                        static_cast<R*>(rho), static_cast<R*>(u));
