@@ -596,7 +596,6 @@ olb_b200_status setup_boundaries(olb_b200_lattice* L, const uint8_t* ids, const 
   if (L->bc_values) cudaFree(L->bc_values);
   if (L->bc_u) cudaFree(L->bc_u);
   if (L->bc_base) cudaFree(L->bc_base);
-  if (L->force) cudaFree(L->force);
   L->bc_base = nullptr;
   L->bc_cells = nullptr;
   L->bc_values = nullptr;

@@ -159,3 +159,22 @@ def test_caller_owned_steps_under_graph_capture(storage):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+def test_force_field_outlives_set_dynamics():
+    """The FORCE field stays the lattice's until it is removed: setting the dynamics
+    again neither frees nor forgets it."""
+    rng = np.random.default_rng(6)
+    case = C.with_force_field(C.periodic_case(19, (8, 9, 10), kind=O.FORCED_BGK), np.float32, rng)
+    f0 = C.random_state(19, case.n, np.float32, rng)
+    out = []
+    for again in (False, True):
+        with ob.Lattice(19, case.size, case.periodic) as lat:
+            lat.set_dynamics(C.to_abi_table(case))
+            lat.set_force_field(case.force_field)
+            if again:
+                lat.set_dynamics(C.to_abi_table(case))
+            lat.set_populations(f0)
+            lat.collide_and_stream(4)
+            out.append(lat.get_populations())
+    assert np.array_equal(out[0], out[1])
