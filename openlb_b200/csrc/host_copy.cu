@@ -17,6 +17,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -35,7 +36,8 @@ class Pool {
 public:
   static std::unique_ptr<Pool> make()
   {
-    std::unique_ptr<Pool> p(new Pool);
+    std::unique_ptr<Pool> p(new (std::nothrow) Pool);
+    if (!p) return nullptr;
     void* base = nullptr;
     if (cudaHostAlloc(&base, kRing * kChunk, cudaHostAllocPortable) != cudaSuccess) {
       (void)cudaGetLastError();
@@ -43,7 +45,7 @@ public:
     }
     p->base_ = static_cast<char*>(base);
     const int n = std::max(1, std::min(kMaxThreads, int(std::thread::hardware_concurrency()) - 1));
-    try {
+    try {  // nothing is thrown through the C interface: fewer threads, or the direct copy
       for (int k = 0; k < n; ++k) p->threads_.emplace_back([q = p.get()] { q->work(); });
     } catch (...) {
       if (p->threads_.empty()) return nullptr;
