@@ -652,11 +652,14 @@ olb_b200_status olb_b200_ensemble_add(olb_b200_ensemble* E, const olb_b200_insta
   if (!(d->omega > 0.0 && d->omega < 2.0)) return efail(OLB_B200_ERR_ARG, "ensemble_add: omega outside (0,2)");
   const uint64_t cells = uint64_t(d->nx) * d->ny * d->nz;
   if (table) {
-    for (uint64_t c = 0; c < cells; ++c) {
-      if (d->cells[c] > 2)
-        return efail(OLB_B200_ERR_ARG, "ensemble_add: cell " + std::to_string(c) + " has class " +
-                                         std::to_string(unsigned(d->cells[c])) +
-                                         " (0 fluid, 1 wall, 2 moving wall)");
+    // a pass the compiler vectorises; the offending cell is looked for when there is one
+    uint8_t largest = 0;
+    for (uint64_t c = 0; c < cells; ++c) largest = std::max(largest, d->cells[c]);
+    if (largest > 2) {
+      uint64_t c = 0;
+      while (d->cells[c] <= 2) ++c;
+      return efail(OLB_B200_ERR_ARG, "ensemble_add: cell " + std::to_string(c) + " has class " +
+                                       std::to_string(unsigned(d->cells[c])) + " (0 fluid, 1 wall, 2 moving wall)");
     }
   }
   // the step kernel indexes an instance's populations with 32 bits

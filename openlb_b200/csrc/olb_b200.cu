@@ -387,7 +387,13 @@ void compute_bulk_box(olb_b200_lattice* L, const uint8_t* ids, int bulk_entry)
   for (int d = 0; d < 3; ++d) g.bulk_lo[d] = g.bulk_hi[d] = 0;
   if (!ids || bulk_entry < 0) return;
   const int n[3] = {L->desc.nx, L->desc.ny, L->desc.nz};
-  auto id_at = [&](int x, int y, int z) { return int(ids[(size_t(x) * n[1] + y) * n[2] + z]); };
+  // whether every cell of row (x, y) in [z0, z1) uses the bulk entry
+  auto row_clean = [&](int x, int y, int z0, int z1) {
+    const uint8_t* row = ids + (size_t(x) * n[1] + y) * n[2];
+    uint8_t other = 0;
+    for (int z = z0; z < z1; ++z) other |= uint8_t(row[z] ^ uint8_t(bulk_entry));
+    return other == 0;
+  };
   int lo[3] = {0, 0, 0}, hi[3] = {n[0], n[1], n[2]};
   auto face_clean = [&](int axis, int layer) {
     int a[3], b[3];
@@ -396,8 +402,7 @@ void compute_bulk_box(olb_b200_lattice* L, const uint8_t* ids, int bulk_entry)
     b[axis] = layer + 1;
     for (int x = a[0]; x < b[0]; ++x)
       for (int y = a[1]; y < b[1]; ++y)
-        for (int z = a[2]; z < b[2]; ++z)
-          if (id_at(x, y, z) != bulk_entry) return false;
+        if (!row_clean(x, y, a[2], b[2])) return false;
     return true;
   };
   for (bool changed = true; changed;) {
@@ -411,15 +416,17 @@ void compute_bulk_box(olb_b200_lattice* L, const uint8_t* ids, int bulk_entry)
   // the bounding box of the other entries inside the box
   int olo[3] = {hi[0], hi[1], hi[2]}, ohi[3] = {lo[0] - 1, lo[1] - 1, lo[2] - 1};
   for (int x = lo[0]; x < hi[0]; ++x)
-    for (int y = lo[1]; y < hi[1]; ++y)
+    for (int y = lo[1]; y < hi[1]; ++y) {
+      if (row_clean(x, y, lo[2], hi[2])) continue;
       for (int z = lo[2]; z < hi[2]; ++z)
-        if (id_at(x, y, z) != bulk_entry) {
+        if (ids[(size_t(x) * n[1] + y) * n[2] + z] != bulk_entry) {
           const int p[3] = {x, y, z};
           for (int d = 0; d < 3; ++d) {
             olo[d] = std::min(olo[d], p[d]);
             ohi[d] = std::max(ohi[d], p[d]);
           }
         }
+    }
   if (ohi[0] >= lo[0]) {
     // six slabs beside the obstacles: below olo[d] or above ohi[d] along axis d
     size_t best = 0;
@@ -618,6 +625,11 @@ olb_b200_status setup_boundaries(olb_b200_lattice* L, const uint8_t* ids, const 
   std::vector<uint32_t> flat, edges, corners, local;
   for (int x = 0; x < nx; ++x) {
     for (int y = 0; y < ny; ++y) {
+      // a row of one entry without values is passed over as a whole
+      const uint8_t* row = ids + (size_t(x) * ny + y) * nz;
+      uint8_t other = 0;
+      for (int z = 0; z < nz; ++z) other |= uint8_t(row[z] ^ row[0]);
+      if (other == 0 && !has_values(table[row[0]].kind)) continue;
       for (int z = 0; z < nz; ++z) {
         const size_t c = (size_t(x) * ny + y) * nz + z;
         const int k = ids[c];
@@ -911,11 +923,17 @@ olb_b200_status olb_b200_set_dynamics(olb_b200_lattice* L, const uint8_t* ids,
   uint8_t first = 0;
   if (ids) {
     first = ids[0];
-    uniform = true;
+    // a pass the compiler vectorises; the offending cell is looked for when there is one
+    uint8_t largest = 0, other = 0;
     for (size_t c = 0; c < L->cells; ++c) {
-      if (ids[c] >= n_entries)
-        return fail(OLB_B200_ERR_ARG, "set_dynamics: cell %zu has id %u >= %d entries", c, unsigned(ids[c]), n_entries);
-      uniform &= ids[c] == first;
+      largest = std::max(largest, ids[c]);
+      other |= uint8_t(ids[c] ^ first);
+    }
+    uniform = other == 0;
+    if (largest >= n_entries) {
+      size_t c = 0;
+      while (ids[c] < n_entries) ++c;
+      return fail(OLB_B200_ERR_ARG, "set_dynamics: cell %zu has id %u >= %d entries", c, unsigned(ids[c]), n_entries);
     }
   }
   olb_b200_status st = select_device(L);
