@@ -778,8 +778,11 @@ OLB_DEV bool collide_any(float (&f)[L::q], int kind, const DynDevice<float>* e, 
 
 // Collision of two cells held as packed 16-bit pairs (low half: cell n_lo of
 // the natural order, high half: cell n_hi), in place; kind and table entry per
-// cell.  count_hi: the high cell enters the statistics.
-template <int Q, class S, int KIND, bool MASKED, bool STATS>
+// cell.  count_hi: the high cell enters the statistics.  KEEP: a cell that passes
+// its populations through (kLanePass) keeps their bits, an infinity or NaN among
+// them with the others untouched; without, it runs as a lane and comes back
+// rounded like a wall lane (see ScaledParams).
+template <int Q, class S, int KIND, bool MASKED, bool STATS, bool KEEP = false>
 OLB_DEV void collide_packed(typename Pair<S>::T (&raw)[Q], const Geometry& g,
                             const DynDevice<float>* __restrict__ table, const DynDevice<float>& bulk, int kind_lo,
                             int kind_hi, int id_lo, int id_hi, uint32_t n_lo, uint32_t n_hi, bool count_hi,
@@ -826,7 +829,8 @@ OLB_DEV void collide_packed(typename Pair<S>::T (&raw)[Q], const Geometry& g,
     lane_lo = mode(kind_lo);
     lane_hi = mode(kind_hi);
     // a moving wall adds its momentum terms: one cell after the other
-    both = kind_lo != K_BOUNCE_BACK_VELOCITY && kind_hi != K_BOUNCE_BACK_VELOCITY;
+    both = KEEP ? lane_lo != kLanePass && lane_hi != kLanePass
+                : kind_lo != K_BOUNCE_BACK_VELOCITY && kind_hi != K_BOUNCE_BACK_VELOCITY;
   }
   if (both) {
     // Both cells at once, in the scaled representation g_i = s_i (f_i - w_i)
@@ -1083,7 +1087,7 @@ OLB_DEV void split_tile(S* __restrict__ pops, const Geometry& g, const DynDevice
     });
     if (!store[0] && !store[1]) return;
   }
-  collide_packed<Q, S, KIND, MASKED, STATS>(raw, g, table, bulk, kind[0], kind[1], id[0], id[1], n[0], n[1], two, acc);
+  collide_packed<Q, S, KIND, MASKED, STATS, true>(raw, g, table, bulk, kind[0], kind[1], id[0], id[1], n[0], n[1], two, acc);
   const Neighbours a(g, int(opaque(uint32_t(x))), int(opaque(uint32_t(y[0]))), int(opaque(uint32_t(z[0])))),
     b(g, int(opaque(uint32_t(x))), int(opaque(uint32_t(y[1]))), int(opaque(uint32_t(z[1]))));
   const uint32_t stride = opaque(g.stride);
