@@ -5,14 +5,24 @@
 // thread, which also takes the page faults of memory the caller has just
 // allocated (every numpy.empty).  Here the copy engine fills a ring of pinned
 // buffers while threads empty it into the destination, each taking its chunk's
-// faults: a chunk of 30 served cavities with their fields, 148 MB into fresh
-// arrays, takes 41 ms instead of 62, 27 of them steps.  Pinned destinations and
+// faults.  268 MB of 256^3 density and velocity on a 16-core host: 16 ms into
+// fresh arrays (57 direct), 8 into arrays used before (16 direct); with two
+// cores 38 (57) and 18 (16).  The fields of 30 served cavities, 148 MB in 60
+// copies: 23 ms fresh (64 direct), 8.3 reused (10.5).  Pinned destinations and
 // small copies go straight to cudaMemcpyAsync; so does a copy that finds the
 // ring taken by another thread.
+//
+// One thread waits for the device: the caller, as with a direct copy.  The copy
+// threads sleep until the first chunk is there, so a copy called behind a long
+// solve keeps one core waiting, not all of theirs.
 #include "host_copy.h"
+
+#include <pthread.h>
+#include <sched.h>
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstring>
 #include <memory>
@@ -25,13 +35,17 @@ namespace olb_b200 {
 namespace {
 
 constexpr size_t kChunk = size_t(512) << 10;
-constexpr int kRing = 16;                        // 8 MiB of pinned memory per process
+constexpr size_t kRing = 16;                     // 8 MiB of pinned memory per process
 constexpr size_t kStagedFrom = size_t(1) << 20;  // below, too few chunks to overlap
 constexpr int kMaxThreads = 6;
+// how long a thread looks for the next chunk (or the caller for a free buffer)
+// before it sleeps: chunks land every 10 us, waking takes several times that
+constexpr std::chrono::microseconds kLook{50};
 
-// One copy at a time (the pool's mutex).  Chunk i passes through buffer
-// i % kRing: the caller issues its transfer once chunk i - kRing has left the
-// buffer, a worker waits for the transfer and writes the chunk out.
+// One copy at a time (Shared::in_use).  Chunk i passes through buffer i % kRing:
+// the caller issues its transfer once chunk i - kRing has left the buffer,
+// waits for the transfers in order and hands out each chunk as it lands; any
+// thread, the caller too when it has nothing to issue or wait for, writes it out.
 class Pool {
 public:
   static std::unique_ptr<Pool> make()
@@ -44,11 +58,11 @@ public:
       return nullptr;
     }
     p->base_ = static_cast<char*>(base);
-    const int n = std::max(1, std::min(kMaxThreads, int(std::thread::hardware_concurrency()) - 1));
-    try {  // nothing is thrown through the C interface: fewer threads, or the direct copy
-      for (int k = 0; k < n; ++k) p->threads_.emplace_back([q = p.get()] { q->work(); });
+    cpu_set_t cpus;
+    const int n = sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : 1;
+    try {  // nothing is thrown through the C interface: fewer threads, the caller writes the rest
+      for (int k = 0; k < std::min(kMaxThreads, n - 1); ++k) p->threads_.emplace_back([q = p.get()] { q->work(); });
     } catch (...) {
-      if (p->threads_.empty()) return nullptr;
     }
     return p;
   }
@@ -69,8 +83,12 @@ public:
   {
     if (device != events_device_) {  // events belong to a device
       drop_events();
+      unsigned flags = 0;  // the caller waits as it has asked to wait for this device
+      if (cudaGetDeviceFlags(&flags) != cudaSuccess) (void)cudaGetLastError();
+      const bool sleep = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
       for (cudaEvent_t& ev : events_) {
-        const cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        const cudaError_t e =
+          cudaEventCreateWithFlags(&ev, cudaEventDisableTiming | (sleep ? cudaEventBlockingSync : 0));
         if (e != cudaSuccess) {
           drop_events();
           return e;
@@ -78,7 +96,44 @@ public:
       }
       events_device_ = device;
     }
-    return run(dst, src, bytes, device, stream);
+    const size_t chunks = (bytes + kChunk - 1) / kChunk;
+    size_t issued = 0;
+    cudaError_t e = cudaSuccess;
+    std::unique_lock<std::mutex> lock(mutex_);
+    dst_ = dst;
+    bytes_ = bytes;
+    taken_ = 0;
+    landed_ = 0;
+    written_ = 0;
+    for (size_t& l : left_) l = 0;
+    while (landed_ < chunks && e == cudaSuccess) {
+      const size_t b = issued % kRing;
+      if (issued < chunks && issued < landed_ + kRing && left_[b] == issued / kRing) {
+        const size_t at = issued++ * kChunk;
+        lock.unlock();
+        e = cudaMemcpyAsync(base_ + b * kChunk, src + at, std::min(kChunk, bytes - at), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaEventRecord(events_[b], stream);
+        lock.lock();
+      } else if (landed_ < issued) {
+        lock.unlock();
+        e = cudaEventSynchronize(events_[landed_ % kRing]);
+        lock.lock();
+        if (e == cudaSuccess) {
+          if (++landed_ == 1) wake_.notify_all();
+          else wake_.notify_one();
+        }
+      } else if (!write_one(lock)) {
+        const size_t seen = written_;
+        wait(lock, freed_, [&] { return written_ != seen; });
+      }
+    }
+    while (write_one(lock)) {}
+    wait(lock, freed_, [&] { return written_ == landed_; });
+    if (e != cudaSuccess) {  // no transfer may reach the ring after the copy
+      lock.unlock();
+      cudaStreamSynchronize(stream);
+    }
+    return e;
   }
 
 private:
@@ -93,87 +148,56 @@ private:
     events_device_ = -1;
   }
 
-  cudaError_t run(char* dst, const char* src, size_t bytes, int device, cudaStream_t stream)
+  // waits for `there` (atomics only): looks for a while, then sleeps
+  template <class F>
+  static void wait(std::unique_lock<std::mutex>& lock, std::condition_variable& cv, F&& there)
   {
-    const size_t chunks = (bytes + kChunk - 1) / kChunk;
-    {
-      std::lock_guard<std::mutex> lock(mutex_);
-      dst_ = dst;
-      bytes_ = bytes;
-      device_ = device;
-      chunks_ = chunks;
-      next_ = 0;
-      issued_ = 0;
-      error_ = cudaSuccess;
-      for (auto& l : left_) l = 0;
-      busy_ = int(threads_.size());
-      ++job_;
-    }
-    wake_.notify_all();
-    cudaError_t e = cudaSuccess;
-    for (size_t i = 0; i < chunks && e == cudaSuccess; ++i) {
-      const int b = int(i % kRing);
-      // left_[b] counts the chunks that have left buffer b
-      while (left_[b].load(std::memory_order_acquire) < i / kRing) std::this_thread::yield();
-      const size_t at = i * kChunk;
-      e = cudaMemcpyAsync(base_ + size_t(b) * kChunk, src + at, std::min(kChunk, bytes - at), cudaMemcpyDeviceToHost,
-                          stream);
-      if (e == cudaSuccess) e = cudaEventRecord(events_[b], stream);
-      if (e == cudaSuccess) issued_.store(i + 1, std::memory_order_release);
-    }
-    if (e != cudaSuccess) stop_ = true;  // workers give up the chunks that never come
-    {
-      std::unique_lock<std::mutex> lock(mutex_);
-      idle_.wait(lock, [&] { return busy_ == 0; });
-    }
-    stop_ = false;
-    return e != cudaSuccess ? e : error_.load();
+    if (there()) return;
+    lock.unlock();
+    const auto until = std::chrono::steady_clock::now() + kLook;
+    while (!there() && std::chrono::steady_clock::now() < until) std::this_thread::yield();
+    lock.lock();
+    cv.wait(lock, there);
+  }
+
+  // writes out the next chunk that has landed; false when there is none
+  bool write_one(std::unique_lock<std::mutex>& lock)
+  {
+    if (taken_ == landed_) return false;
+    const size_t i = taken_++, at = i * kChunk;
+    lock.unlock();
+    std::memcpy(dst_ + at, base_ + (i % kRing) * kChunk, std::min(kChunk, bytes_ - at));
+    lock.lock();
+    ++left_[i % kRing];
+    ++written_;
+    return true;
   }
 
   void work()
   {
-    uint64_t seen = 0;
-    for (;;) {
-      {
-        std::unique_lock<std::mutex> lock(mutex_);
-        wake_.wait(lock, [&] { return quit_ || job_ != seen; });
-        if (quit_) return;
-        seen = job_;
+    (void)pthread_setname_np(pthread_self(), "olb-copy");
+    std::unique_lock<std::mutex> lock(mutex_);
+    while (!quit_) {
+      if (write_one(lock)) {
+        freed_.notify_one();
+        continue;
       }
-      cudaSetDevice(device_);
-      for (;;) {
-        const size_t i = next_.fetch_add(1);
-        if (i >= chunks_) break;
-        while (issued_.load(std::memory_order_acquire) <= i && !stop_) std::this_thread::yield();
-        if (issued_.load(std::memory_order_acquire) <= i) break;
-        const int b = int(i % kRing);
-        const cudaError_t e = cudaEventSynchronize(events_[b]);
-        const size_t at = i * kChunk;
-        if (e == cudaSuccess) std::memcpy(dst_ + at, base_ + size_t(b) * kChunk, std::min(kChunk, bytes_ - at));
-        else error_ = e;
-        left_[b].fetch_add(1, std::memory_order_release);
-      }
-      std::lock_guard<std::mutex> lock(mutex_);
-      if (--busy_ == 0) idle_.notify_all();
+      wait(lock, wake_, [&] { return quit_ || taken_ != landed_; });
     }
   }
 
   char* base_ = nullptr;
   std::vector<std::thread> threads_;
   std::mutex mutex_;
-  std::condition_variable wake_, idle_;
-  bool quit_ = false;
-  uint64_t job_ = 0;
-  int busy_ = 0;
-  // the current copy
-  char* dst_ = nullptr;
-  size_t bytes_ = 0, chunks_ = 0;
-  int device_ = 0;
+  std::condition_variable wake_, freed_;  // chunks to write; a chunk written
+  std::atomic<bool> quit_{false};
   cudaEvent_t events_[kRing] = {};
   int events_device_ = -1;
-  std::atomic<size_t> next_{0}, issued_{0}, left_[kRing];
-  std::atomic<cudaError_t> error_{cudaSuccess};
-  std::atomic<bool> stop_{false};
+  // the current copy (mutex_; the atomics are also looked at without it)
+  char* dst_ = nullptr;
+  size_t bytes_ = 0;
+  size_t left_[kRing] = {};                                  // chunks that have left each buffer
+  std::atomic<size_t> landed_{0}, taken_{0}, written_{0};  // chunks in the ring so far, taken by a thread, written out
 };
 
 // holders, the pool and its use; never destroyed (a handle leaked at exit

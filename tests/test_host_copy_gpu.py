@@ -2,7 +2,11 @@
 same results copied into pinned memory (one direct copy)."""
 from __future__ import annotations
 
+import subprocess
+import sys
 import threading
+import time
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -69,3 +73,60 @@ def test_threads_with_their_own_lattices():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_a_copy_behind_a_solve_keeps_one_core_waiting():
+    """get_moments called with a third of a second of steps still queued: the copy
+    threads sleep until there is something to copy."""
+    with ob.Lattice(19, (256, 256, 256), (True,) * 3) as lat:
+        lat.set_dynamics([ob.BGKdynamics(omega=1.3)])
+        lat.ini_equilibrium(np.ones(lat.n, np.float32), np.zeros((3, lat.n), np.float32))
+        out = lat.get_moments()
+        for _ in range(2):
+            lat.get_moments(out=out)
+        steps = int(350 / (lat.time_steps(20) / 20))
+        assert steps < 1000  # all of them queued at once
+        cpu, wall = time.process_time(), time.perf_counter()
+        lat.collide_and_stream(steps)
+        lat.get_moments(out=out)
+        cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
+        # the waiting caller is 1; seven threads for the 8 ms of the copy add under 0.2
+        assert wall > 0.3 and cpu / wall < 1.5, (cpu, wall)
+
+
+# a program that asks for waits that sleep (cudaDeviceScheduleBlockingSync)
+SLEEPING = """
+import ctypes, sys, time
+assert ctypes.CDLL("libcuda.so.1").cuInit(0) == 0
+assert ctypes.CDLL("libcuda.so.1").cuDevicePrimaryCtxSetFlags_v2(0, 4) == 0
+import numpy as np
+import openlb_b200 as ob
+with ob.Lattice(27, (192, 192, 192), (True,) * 3, storage="f64") as lat:  # half a millisecond a step
+    lat.set_dynamics([ob.BGKdynamics(omega=1.3)])
+    lat.ini_equilibrium(np.ones(lat.n), np.zeros((3, lat.n)))
+    out = lat.get_moments()
+    lat.get_moments(out=out)
+    lat.collide_and_stream(2, stats=True)
+    steps = int(400 / (lat.time_steps(20) / 20))
+    assert steps < 1000  # all of them queued at once
+    cpu, wall = time.process_time(), time.perf_counter()
+    if sys.argv[1] == "copy":
+        lat.collide_and_stream(steps)
+        lat.get_moments(out=out)
+    else:
+        lat.collide_and_stream(steps, stats=True)
+    print(time.process_time() - cpu, time.perf_counter() - wall)
+"""
+
+
+def cpu_and_wall_of_a_sleeping_wait(what):
+    r = subprocess.run([sys.executable, "-c", SLEEPING, what], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parents[1])
+    assert r.returncode == 0, r.stderr[-2000:]
+    return (float(v) for v in r.stdout.split())
+
+
+def test_a_program_whose_waits_sleep_sleeps_behind_a_solve():
+    cpu, wall = cpu_and_wall_of_a_sleeping_wait("copy")
+    # 0.1 s of processor time at most for enqueueing and for seven threads' part of 226 MB
+    assert wall > 0.3 and cpu < 0.5 * wall, (cpu, wall)
