@@ -9,7 +9,7 @@ namespace olb_b200 {
 
 // A handle that copies results out holds one of these for its lifetime.  All
 // holders of a process share one set of staging buffers and copy threads, made
-// by the first large copy and given back with the last holder.
+// once they have copied a good deal and given back with the last holder.
 class HostCopyHold {
 public:
   HostCopyHold();

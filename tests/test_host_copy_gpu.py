@@ -2,6 +2,7 @@
 same results copied into pinned memory (one direct copy)."""
 from __future__ import annotations
 
+import os
 import subprocess
 import sys
 import threading
@@ -15,6 +16,25 @@ import openlb_b200 as ob
 from tests import cases as C
 
 pytestmark = pytest.mark.gpu
+
+
+def copy_threads():
+    """The library's copy threads alive in this process."""
+    names = []
+    for task in os.listdir("/proc/self/task"):
+        try:
+            names.append(Path("/proc/self/task", task, "comm").read_text().strip())
+        except FileNotFoundError:  # it ended meanwhile
+            pass
+    return names.count("olb-copy")
+
+
+def make_staged(lat):
+    """Copies of 1 MiB and more take the staged way once 32 MiB have gone directly."""
+    out = lat.get_moments()
+    for _ in range((32 << 20) // (3 * 4 * lat.n) + 1):
+        lat.get_moments(out=out)
+    assert copy_threads() > 0
 
 
 def pinned(lat):
@@ -35,6 +55,7 @@ def test_pageable_equals_pinned(size):
                             (0.03 * rng.standard_normal((3, n))).astype(np.float32))
         lat.collide_and_stream(3)
         want = pinned(lat)
+        make_staged(lat)
         for _ in range(3):
             got = lat.get_moments()
             assert np.array_equal(got[0], want[0]) and np.array_equal(got[1].reshape(-1), want[1].reshape(-1))
@@ -68,11 +89,33 @@ def test_threads_with_their_own_lattices():
             errors.append((k, repr(e)))
 
     threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
-    for t in threads:
-        t.start()
-    for t in threads:
-        t.join()
+    with ob.Lattice(19, (8, 64, 511), (True,) * 3) as lat:
+        make_staged(lat)
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
     assert not errors, errors
+
+
+def test_small_solves_make_no_ring():
+    """A handle per solve: neither pinned buffers nor threads until the handles alive
+    have copied 32 MiB, and none left when the last one is closed."""
+    assert copy_threads() == 0
+    for _ in range(4):  # 14 MB each
+        with ob.Lattice(19, (96, 96, 96), (True,) * 3) as lat:
+            lat.set_dynamics([ob.BGKdynamics(omega=1.3)])
+            lat.get_moments()
+            assert copy_threads() == 0
+    with ob.Lattice(19, (96, 96, 96), (True,) * 3) as lat:
+        lat.set_dynamics([ob.BGKdynamics(omega=1.3)])
+        for _ in range(3):
+            lat.get_moments()
+        assert copy_threads() > 0
+        with ob.Lattice(19, (8, 8, 8), (True,) * 3):
+            pass
+        assert copy_threads() > 0
+    assert copy_threads() == 0
 
 
 def test_a_copy_behind_a_solve_keeps_one_core_waiting():
