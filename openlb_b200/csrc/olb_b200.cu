@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -479,7 +480,9 @@ StatSink stat_sink(olb_b200_lattice* L, size_t blocks, bool in_kernel)
 // Reduces `count` partials into stat_host unless their kernel did (reduced),
 // and waits for the result.  The device writes it into pinned memory with its
 // number last; the host polls for that number, which costs less than a copy
-// and a synchronisation, and looks at the stream's state now and then.
+// and a synchronisation, for up to kPoll.  A result further off (many steps in
+// the call, or an error) is waited for as the program has asked to wait for the
+// device.
 olb_b200_status finish_stats(olb_b200_lattice* L, size_t count, bool reduced)
 {
   const unsigned long long seq = ++L->stat_seq;
@@ -489,11 +492,12 @@ olb_b200_status finish_stats(olb_b200_lattice* L, size_t count, bool reduced)
                                          L->partials, count, L->stat_stage, L->stat_host, seq);
     if (e != cudaSuccess) return cuda_fail(e, "statistics reduction launch");
   }
+  constexpr std::chrono::milliseconds kPoll{1};
   const volatile unsigned long long* done = &L->stat_host->seq;
+  const auto until = std::chrono::steady_clock::now() + kPoll;
   for (unsigned polls = 1; *done != seq; ++polls) {
-    if (polls % 4096) continue;
-    const cudaError_t e = cudaStreamQuery(L->stream);
-    if (e == cudaErrorNotReady) continue;
+    if (polls % 1024 || std::chrono::steady_clock::now() < until) continue;
+    const cudaError_t e = cudaStreamSynchronize(L->stream);
     if (e != cudaSuccess) return cuda_fail(e, "statistics");
     if (*done != seq) return fail(OLB_B200_ERR_CUDA, "statistics: the reduction left no result");
   }

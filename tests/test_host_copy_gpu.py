@@ -173,3 +173,9 @@ def test_a_program_whose_waits_sleep_sleeps_behind_a_solve():
     cpu, wall = cpu_and_wall_of_a_sleeping_wait("copy")
     # 0.1 s of processor time at most for enqueueing and for seven threads' part of 226 MB
     assert wall > 0.3 and cpu < 0.5 * wall, (cpu, wall)
+
+
+def test_a_program_whose_waits_sleep_sleeps_for_statistics():
+    cpu, wall = cpu_and_wall_of_a_sleeping_wait("statistics")
+    # under 0.1 s for enqueueing and a millisecond of polling
+    assert wall > 0.3 and cpu < 0.5 * wall, (cpu, wall)
