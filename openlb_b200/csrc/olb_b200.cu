@@ -325,9 +325,8 @@ int cells_per_thread(const olb_b200_lattice* L)
 // shape is fixed.
 void choose_tiles(olb_b200_lattice* L)
 {
-  const bool only_flat = L->elem == 2 && !L->g.paired && kSplitNatural16;
   L->g.flat = 0;
-  if (only_flat || !L->shape_fixed || L->flat_fixed) set_flat(L->g, flat_threads(int(L->elem)));
+  if (!L->shape_fixed || L->flat_fixed) set_flat(L->g, flat_threads(int(L->elem)));
 }
 
 // The geometry a step launches with.  Steps that reduce statistics use blocks
@@ -1435,7 +1434,6 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
         L->block_z = bz;
         L->block_y = kStepThreads / bz;
         L->g.flat = 0;
-        if (L->elem == 2 && !L->g.paired && kSplitNatural16) continue;  // flat tiles only
       }
       st = enqueue_steps(L, 2, false);  // warm-up
       if (st != OLB_B200_OK) break;
