@@ -321,6 +321,13 @@ int cells_per_thread(const olb_b200_lattice* L)
   return step_cells(L->g, int(L->elem), L->variant);
 }
 
+// What runs when variant v is selected: the natural 16-bit layout has one kernel
+StepVariant running_variant(const olb_b200_lattice* L, int v)
+{
+  if (L->elem == 2 && !L->g.paired && kSplitNatural16) return StepVariant{2, kSplitMinBlocks};
+  return step_variant(int(L->elem), v);
+}
+
 // How the step kernels cut a plane: flat tiles (flat_threads) unless a launch
 // shape is fixed.
 void choose_tiles(olb_b200_lattice* L)
@@ -1381,8 +1388,9 @@ olb_b200_status olb_b200_get_tuning(olb_b200_lattice* L, olb_b200_tuning* out)
 {
   if (!L || !out) return fail(OLB_B200_ERR_ARG, "get_tuning: null argument");
   out->variant = L->variant;
-  out->cells_per_thread = cells_per_thread(L);
-  out->min_blocks_per_sm = step_variant(int(L->elem), L->variant).min_blocks;
+  const StepVariant running = running_variant(L, L->variant);
+  out->cells_per_thread = running.cells_per_thread;
+  out->min_blocks_per_sm = running.min_blocks;
   out->block_z = L->block_z;
   out->block_y = L->block_y;
   out->tuned = L->tuned ? 1 : 0;
@@ -1418,7 +1426,7 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
   for (int v = 0; v < kNumStepVariants && st == OLB_B200_OK; ++v) {
     bool duplicate = false;
     for (int w = 0; w < v; ++w) {
-      const StepVariant a = step_variant(int(L->elem), v), b = step_variant(int(L->elem), w);
+      const StepVariant a = running_variant(L, v), b = running_variant(L, w);
       duplicate |= a.cells_per_thread == b.cells_per_thread && a.min_blocks == b.min_blocks;
     }
     if (duplicate) continue;

@@ -232,3 +232,19 @@ def test_a_launch_shape_is_what_runs(storage, nx):
             out.append(lat.get_populations())
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
     assert len(sums) == 3
+
+
+# launch shapes timed at nz = 75: 64x4, 32x8 and flat tiles
+@pytest.mark.parametrize("storage,nx,kernels", [
+    ("f16", 5, [(2, 3)] * 4),                              # the natural layout's one kernel
+    ("f16", 6, [(1, 3), (1, 4), (1, 3), (1, 4)]),          # one element per thread
+    ("f32", 5, [(1, 3), (1, 4), (2, 2), (2, 3)]),
+])
+def test_tuning_reports_the_kernel_that_runs(storage, nx, kernels):
+    with ob.Lattice(19, (nx, 20, 75), (True,) * 3, storage=storage) as lat:
+        lat.set_dynamics([ob.BGKdynamics(omega=1.3)])
+        for variant, kernel in enumerate(kernels):
+            lat.set_step_variant(variant)
+            t = lat.tuning()
+            assert (t["variant"], t["cells_per_thread"], t["min_blocks_per_sm"]) == (variant,) + kernel
+        assert lat.autotune(2)["candidates"] == 3 * len(set(kernels))
