@@ -263,8 +263,9 @@ struct olb_b200_lattice {
   unsigned long long stat_seq = 0;   // number of the last reduction
   int block_z = 0, block_y = 0;
   int variant = 0;          // index of the step-kernel variant (step_variant)
-  bool shape_fixed = false; // block_z, block_y (or flat tiles) chosen by the caller or the autotuner
-  bool flat_fixed = false;  // the autotuner chose flat tiles
+  // block_z, block_y: the default (flat tiles), a rectangle set by the caller, or
+  // what the autotuner chose
+  enum Shape { kDefaultShape, kCallersShape, kTunedRectangle, kTunedFlat } shape = kDefaultShape;
   void* force = nullptr;    // FORCE per cell, 3 columns of `stride` R (olb_b200_set_force_field)
   bool tuned = false;       // variant and shape chosen by olb_b200_autotune
   float tuned_ms = 0.f;
@@ -333,7 +334,18 @@ StepVariant running_variant(const olb_b200_lattice* L, int v)
 void choose_tiles(olb_b200_lattice* L)
 {
   L->g.flat = 0;
-  if (!L->shape_fixed || L->flat_fixed) set_flat(L->g, flat_threads(int(L->elem)));
+  if (L->shape == olb_b200_lattice::kDefaultShape || L->shape == olb_b200_lattice::kTunedFlat) set_flat(L->g, flat_threads(int(L->elem)));
+}
+
+// Forgets what the autotuner chose, its launch shape too.
+void drop_tuning(olb_b200_lattice* L)
+{
+  L->tuned = false;
+  if (L->shape == olb_b200_lattice::kTunedRectangle || L->shape == olb_b200_lattice::kTunedFlat) {
+    default_shape(L, L->block_z, L->block_y);
+    L->shape = olb_b200_lattice::kDefaultShape;
+    choose_tiles(L);
+  }
 }
 
 // The geometry a step launches with.  Steps that reduce statistics use blocks
@@ -1002,7 +1014,7 @@ olb_b200_status olb_b200_set_dynamics(olb_b200_lattice* L, const uint8_t* ids,
   // a change of kernel class invalidates an earlier tuning
   if (!L->tuned || was_masked != L->masked) {
     L->variant = default_variant(L);
-    L->tuned = false;
+    drop_tuning(L);
   }
   choose_tiles(L);
   return OLB_B200_OK;
@@ -1224,7 +1236,7 @@ olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* L, int32_t block_z, 
   if (!L) return fail(OLB_B200_ERR_ARG, "set_launch_shape: null lattice");
   if (block_z == 0 && block_y == 0) {
     default_shape(L, L->block_z, L->block_y);
-    L->shape_fixed = L->flat_fixed = false;
+    L->shape = olb_b200_lattice::kDefaultShape;
     choose_tiles(L);
     return OLB_B200_OK;
   }
@@ -1233,8 +1245,7 @@ olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* L, int32_t block_z, 
                 "of 32, block_z*block_y <= %d", block_z, block_y, kStepThreads);
   L->block_z = block_z;
   L->block_y = block_y;
-  L->shape_fixed = true;
-  L->flat_fixed = false;
+  L->shape = olb_b200_lattice::kCallersShape;
   choose_tiles(L);
   return OLB_B200_OK;
 }
@@ -1379,8 +1390,7 @@ olb_b200_status olb_b200_set_step_variant(olb_b200_lattice* L, int32_t variant)
   if (variant < -1 || variant >= kNumStepVariants)
     return fail(OLB_B200_ERR_ARG, "set_step_variant: variant %d outside [-1, %d)", variant, kNumStepVariants);
   L->variant = variant < 0 ? default_variant(L) : variant;
-  L->tuned = false;
-  choose_tiles(L);
+  drop_tuning(L);
   return OLB_B200_OK;
 }
 
@@ -1479,8 +1489,7 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
   L->variant = best_v;
   L->block_z = best_bz;
   L->block_y = best_by;
-  L->shape_fixed = true;
-  L->flat_fixed = best_flat;
+  L->shape = best_flat ? olb_b200_lattice::kTunedFlat : olb_b200_lattice::kTunedRectangle;
   choose_tiles(L);
   L->tuned = true;
   L->tuned_ms = best;

@@ -248,3 +248,25 @@ def test_tuning_reports_the_kernel_that_runs(storage, nx, kernels):
             t = lat.tuning()
             assert (t["variant"], t["cells_per_thread"], t["min_blocks_per_sm"]) == (variant,) + kernel
         assert lat.autotune(2)["candidates"] == 3 * len(set(kernels))
+
+
+@pytest.mark.parametrize("drop", ["set_dynamics", "set_step_variant"])
+def test_a_dropped_tuning_takes_its_launch_shape_along(drop):
+    """What the autotuner chose for one kernel class is not left to another: the lattice
+    is as one that was never tuned.  (Several sizes: the tuner may choose the default.)"""
+    walls = [ob.BGKdynamics(omega=1.3), ob.BounceBack()]
+    for nz in (64, 100, 128, 192, 250, 256, 300, 384):
+        size = (16, 24, nz)
+        ids = (np.arange(16 * 24 * nz) % 5 == 0).astype(np.uint8)
+        seen = []
+        for tune in (False, True):
+            with ob.Lattice(19, size, (True,) * 3) as lat:
+                lat.set_dynamics([walls[0]])
+                if tune:
+                    assert lat.autotune(2)["tuned"]
+                if drop == "set_dynamics":
+                    lat.set_dynamics(walls, ids)
+                else:
+                    lat.set_step_variant(1)
+                seen.append(lat.tuning())
+        assert not seen[1]["tuned"] and seen[0] == seen[1], (nz, seen)
