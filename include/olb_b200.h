@@ -276,7 +276,8 @@ olb_b200_status olb_b200_get_info(olb_b200_lattice* lattice, int64_t* steps_done
 /* Launch shape of the step kernel (threads along z and y, product <= 256,
  * block_z a multiple of 32).  0,0 selects the built-in default: blocks of
  * consecutive cells of a plane's y-z index, which leave no lane without a cell
- * whatever the extents (olb_b200_get_info then reports the nearest rectangle). */
+ * whatever the extents; olb_b200_get_info and olb_b200_get_tuning report them as
+ * (threads, 1).  Steps with statistics launch 256 threads there. */
 olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* lattice, int32_t block_z, int32_t block_y);
 
 /* Step-kernel tuning.  The library compiles a few variants of the step kernel

@@ -1225,8 +1225,9 @@ olb_b200_status olb_b200_get_info(olb_b200_lattice* L, int64_t* steps_done, int6
   if (!L) return fail(OLB_B200_ERR_ARG, "get_info: null lattice");
   if (steps_done) *steps_done = L->steps_done;
   if (device_bytes) *device_bytes = int64_t(L->device_bytes + L->n_partials * sizeof(StatPartial));
-  if (block_z) *block_z = L->block_z;
-  if (block_y) *block_y = L->block_y;
+  const dim3 block = step_block(L->g, L->block_z, L->block_y);
+  if (block_z) *block_z = int32_t(block.x);
+  if (block_y) *block_y = int32_t(block.y);
   return OLB_B200_OK;
 }
 
@@ -1401,8 +1402,9 @@ olb_b200_status olb_b200_get_tuning(olb_b200_lattice* L, olb_b200_tuning* out)
   const StepVariant running = running_variant(L, L->variant);
   out->cells_per_thread = running.cells_per_thread;
   out->min_blocks_per_sm = running.min_blocks;
-  out->block_z = L->block_z;
-  out->block_y = L->block_y;
+  const dim3 block = step_block(L->g, L->block_z, L->block_y);
+  out->block_z = int32_t(block.x);
+  out->block_y = int32_t(block.y);
   out->tuned = L->tuned ? 1 : 0;
   out->candidates = 0;
   out->ms_per_step = L->tuned ? L->tuned_ms : 0.f;

@@ -270,3 +270,21 @@ def test_a_dropped_tuning_takes_its_launch_shape_along(drop):
                     lat.set_step_variant(1)
                 seen.append(lat.tuning())
         assert not seen[1]["tuned"] and seen[0] == seen[1], (nz, seen)
+
+
+@pytest.mark.parametrize("storage,nx,threads", [("f32", 5, 256), ("f64", 6, 256), ("f16", 5, 64), ("bf16", 6, 64)])
+@pytest.mark.parametrize("nz", [9, 75, 300])
+def test_the_reported_block_is_the_one_launched(storage, nx, threads, nz):
+    with ob.Lattice(19, (nx, 20, nz), (True,) * 3, storage=storage) as lat:
+        lat.set_dynamics([ob.BGKdynamics(omega=1.3)])
+
+        def reported():
+            info, tuning = lat.info(), lat.tuning()
+            assert (info["block_z"], info["block_y"]) == (tuning["block_z"], tuning["block_y"])
+            return info["block_z"], info["block_y"]
+
+        assert reported() == (threads, 1)  # flat tiles
+        lat.set_launch_shape(32, 4)
+        assert reported() == (32, 4)
+        lat.set_launch_shape(0, 0)
+        assert reported() == (threads, 1)
