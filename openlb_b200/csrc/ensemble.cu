@@ -242,6 +242,7 @@ ensemble_check_kernel(float* __restrict__ pool, const InstanceDevice* __restrict
                       ResidualPartial* __restrict__ partials)
 {
   using L = L19;
+  static_assert(kTileCells == 1, "a thread checks one cell");
   const int t = blockIdx.x;
   if (t >= *ntiles_ptr) return;
   __shared__ double sh[2][kEnsembleThreads / 32];
@@ -399,7 +400,7 @@ struct olb_b200_ensemble {
   std::vector<Region> free_list;               // sorted by offset
   Tile* tiles_dev = nullptr;
   int max_tiles = 0;
-  int* counts_dev = nullptr;                   // [0] ntiles, [1] ninst
+  int* ntiles_dev = nullptr;
   int* tile_begin_dev = nullptr;
   int* tile_end_dev = nullptr;
   ResidualPartial* partials = nullptr;
@@ -525,11 +526,11 @@ olb_b200_status upload_tables(olb_b200_ensemble* E)
       E->step_grid = bucket;
     }
   }
-  const int counts[2] = {int(tiles.size()), E->max_instances};
+  const int ntiles = int(tiles.size());
   if (!tiles.empty()) {
     OLB_ECUDA(cudaMemcpyAsync(E->tiles_dev, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, E->stream));
   }
-  OLB_ECUDA(cudaMemcpyAsync(E->counts_dev, counts, sizeof counts, cudaMemcpyHostToDevice, E->stream));
+  OLB_ECUDA(cudaMemcpyAsync(E->ntiles_dev, &ntiles, sizeof ntiles, cudaMemcpyHostToDevice, E->stream));
   OLB_ECUDA(cudaMemcpyAsync(E->tile_begin_dev, begin.data(), begin.size() * sizeof(int), cudaMemcpyHostToDevice, E->stream));
   OLB_ECUDA(cudaMemcpyAsync(E->tile_end_dev, end.data(), end.size() * sizeof(int), cudaMemcpyHostToDevice, E->stream));
   OLB_ECUDA(cudaMemcpyAsync(E->table_dev, E->table.data(), E->table.size() * sizeof(InstanceDevice),
@@ -547,11 +548,11 @@ olb_b200_status enqueue_chunk(olb_b200_ensemble* E, int steps, int check)
                         : E->min_blocks == 4 ? ensemble_step_kernel<4>
                                              : ensemble_step_kernel<3>;
     OLB_ECUDA(launch_chained(kernel, k > 0, dim3(unsigned(E->step_grid)), dim3(kEnsembleThreads), E->stream, E->pool,
-                             E->table_dev, E->tiles_dev, E->counts_dev, k));
+                             E->table_dev, E->tiles_dev, E->ntiles_dev, k));
   }
   if (check) {
     ensemble_check_kernel<<<E->step_grid, kEnsembleThreads, 0, E->stream>>>(E->pool, E->table_dev, E->tiles_dev,
-                                                                       E->counts_dev, steps, E->partials);
+                                                                       E->ntiles_dev, steps, E->partials);
     OLB_ECUDA(cudaGetLastError());
   }
   ensemble_finish_kernel<<<E->max_instances, kFinishThreads, 0, E->stream>>>(
@@ -599,7 +600,7 @@ olb_b200_status olb_b200_ensemble_create(const olb_b200_ensemble_desc* desc, olb
   OLB_ECUDA_C(cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking));
   OLB_ECUDA_C(cudaMalloc(&E->pool, E->pool_elems * sizeof(float)));
   OLB_ECUDA_C(cudaMalloc(&E->table_dev, size_t(E->max_instances) * sizeof(InstanceDevice)));
-  OLB_ECUDA_C(cudaMalloc(&E->counts_dev, 2 * sizeof(int)));
+  OLB_ECUDA_C(cudaMalloc(&E->ntiles_dev, sizeof(int)));
   OLB_ECUDA_C(cudaMalloc(&E->tile_begin_dev, size_t(E->max_instances) * sizeof(int)));
   OLB_ECUDA_C(cudaMalloc(&E->tile_end_dev, size_t(E->max_instances) * sizeof(int)));
   OLB_ECUDA_C(cudaMalloc(&E->residual_dev, size_t(E->max_instances) * sizeof(double)));
@@ -625,7 +626,7 @@ void olb_b200_ensemble_destroy(olb_b200_ensemble* E)
   cudaFree(E->pool);
   cudaFree(E->table_dev);
   cudaFree(E->tiles_dev);
-  cudaFree(E->counts_dev);
+  cudaFree(E->ntiles_dev);
   cudaFree(E->tile_begin_dev);
   cudaFree(E->tile_end_dev);
   cudaFree(E->partials);

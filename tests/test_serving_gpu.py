@@ -250,3 +250,33 @@ def test_geometry_table_is_checked():
         assert ens.info()["active"] == 0
     finally:
         ens.close()
+
+
+def test_residuals_of_a_mix_against_the_fields():
+    """Each check's residual against the change of the fetched fields since the check
+    before, in FP64, with the number of steps: instances of one tile up to 500 (the
+    reduction takes 128 a pass), checks at both parities, one admitted later.
+
+    Both sides derive u from the same populations in FP32; contracted differently they
+    differ by a few 2^-24 |u|, so the residuals by less than 1e-6."""
+    sides, chunks = (6, 20, 32, 33, 50), (41, 30, 25)
+    reqs = []
+    for k, n in enumerate(sides):
+        reqs.append(serving.Request(k, 0.0, n, 40.0 + 30.0 * k, 0.1, kind=_abi.ENSEMBLE_GEOMETRY))
+        reqs[-1].geometry = cavity((n, n, n))
+    ens = serving.Ensemble(1 << 28, 8)
+    try:
+        slots, before, done = {}, {}, {}
+        for c, steps in enumerate(chunks):
+            for k in ([0, 1, 2, 4] if c == 0 else [3] if c == 1 else []):
+                slots[k], before[k], done[k] = ens.add(reqs[k]), 0.0, 0
+            residual, counts = ens.run(steps, check=True)
+            for k, slot in slots.items():
+                fluid = reqs[k].geometry.reshape(-1) == 0
+                u = ens.moments(slot, sides[k])[1][:, fluid].astype(np.float64)
+                want = np.sqrt(((u - before[k]) ** 2).sum() / (u ** 2).sum())
+                before[k], done[k] = u, done[k] + steps
+                assert want > 1e-3 and abs(residual[slot] - want) < 1e-6, (c, k, residual[slot], want)
+                assert counts[slot] == done[k]
+    finally:
+        ens.close()
