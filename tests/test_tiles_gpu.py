@@ -56,6 +56,26 @@ def test_periodic_planes_around_a_block(storage, nx, plane):
     check(case, f0, advance(case, f0, STEPS, storage), storage)
 
 
+@pytest.mark.parametrize("storage", ["f32", "f64"])
+@pytest.mark.parametrize("variant", range(4))
+@pytest.mark.parametrize("plane", PLANES)
+def test_planes_around_a_block_in_every_step_variant(storage, variant, plane):
+    """One and two cells per thread (a second run that is empty, partial, full)."""
+    dtype, rtol = (np.float32, 1e-5) if storage == "f32" else (np.float64, 1e-12)
+    case = C.periodic_case(19, (3,) + plane, kind=O.FORCED_TRT)
+    f0 = C.random_state(19, case.n, dtype, np.random.default_rng(37 + plane[0]))
+    ref = f0.copy()
+    O.step(case, ref, STEPS)
+    with ob.Lattice(19, case.size, case.periodic, storage=storage) as lat:
+        lat.set_dynamics(C.to_abi_table(case))
+        lat.set_step_variant(variant)
+        lat.set_populations(f0)
+        lat.collide_and_stream(STEPS - 1)
+        assert lat.collide_and_stream(1, stats=True)["n_cells"] == case.n
+        rel, _ = C.pop_tolerance_violation(19, lat.get_populations(), ref, rtol)
+    assert rel <= rtol, rel
+
+
 @pytest.mark.parametrize("q,storage,nx", [(19, "f16", 5), (27, "bf16", 5), (19, "f16", 6), (19, "f32", 5)])
 @pytest.mark.parametrize("plane", [(7, 9), (3, 43), (16, 16), (9, 57)])
 def test_cavity_planes_around_a_block(q, storage, nx, plane):

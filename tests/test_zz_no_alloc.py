@@ -11,8 +11,9 @@ same populations and statistics as olb_b200_collide_and_stream on a lattice
 handle with the same input, within the tolerances the parity tests use:
 populations within 1e-5 (FP32), 1e-12 (FP64) or 1e-3 (FP16 storage) of the
 unshifted population, summed density within 1e-7 relative, summed |u|^2 and
-max |u|^2 within 1e-5.  The handle runs the same step-kernel variant and
-launch shape as the no-allocation call.  The call only serves triply periodic
+max |u|^2 within 1e-5.  Both run the default step-kernel variant of the
+lattice, which follows its size, collision and storage; the sizes here lie on
+both sides of every change of it.  The call only serves triply periodic
 lattices; other descriptions are rejected before any device work.  This file
 is collected last so a failure here comes after every other test has run.
 """
@@ -52,27 +53,39 @@ def _scales(q):
     return s
 
 
-@pytest.mark.parametrize("q,storage", [(19, "f32"), (27, "f32"), (19, "f64"), (27, "f16")])
-def test_noalloc_matches_lattice_entry_point(q, storage):
+BGK, FORCED_TRT = ob.BGKdynamics(omega=1.3), ob.ForcedTRTdynamics(omega=1.3, force=(1e-4, -2e-5, 3e-5))
+
+# odd nx: a 16-bit handle then keeps one cell per element, the layout the
+# no-allocation call takes.  FP32 takes {1,3} up to one wave of 148 * 3 * 256 =
+# 113 664 cells, {1,4} above, and {2,3} from 2^21 cells on without a force; FP64
+# {1,3} throughout, 16-bit storage the two-cell kernel of the natural layout.
+SMALL, ABOVE_ONE_WAVE, LARGE = (41, 36, 70), (49, 51, 47), (129, 127, 131)
+
+
+@pytest.mark.parametrize("q,storage,size,dynamics,stats", [
+    (19, "f32", SMALL, BGK, True), (27, "f32", SMALL, BGK, True), (19, "f64", SMALL, BGK, True),
+    (27, "f16", SMALL, BGK, True),
+    (19, "f32", ABOVE_ONE_WAVE, BGK, True), (19, "f32", ABOVE_ONE_WAVE, FORCED_TRT, True),
+    (19, "f32", ABOVE_ONE_WAVE, BGK, False),
+    (19, "f32", LARGE, BGK, True), (19, "f32", LARGE, BGK, False), (19, "f32", LARGE, FORCED_TRT, True),
+    (27, "f32", LARGE, BGK, True), (19, "f64", LARGE, BGK, True), (19, "f16", LARGE, FORCED_TRT, False),
+])
+def test_noalloc_matches_lattice_entry_point(q, storage, size, dynamics, stats):
     import torch
 
-    # odd nx: a 16-bit handle then keeps one cell per element, the layout the
-    # no-allocation call takes
-    size = (41, 36, 70)
     n = size[0] * size[1] * size[2]
     stride = (n + 63) // 64 * 64
     rng = np.random.default_rng(2024 + q)
     compute = np.float64 if storage == "f64" else np.float32
     f0 = _state(q, n, rng, compute)
-    omega = 1.3
     lib = _abi.load()
     w = ob.descriptor(q).w(np.float64)[:, None]
     scale = _scales(q)[:, None]
 
     # existing entry point on a lattice handle
     lat = ob.Lattice(q, size, (True, True, True), storage=storage)
-    lat.set_dynamics([ob.BGKdynamics(omega=omega)])
-    lat.set_step_variant(0)       # the variant the no-allocation call uses
+    lat.set_dynamics([dynamics])
+    lat.set_step_variant(-1)      # the default variant, as the no-allocation call
     lat.set_launch_shape(0, 0)    # the library's default launch shape
     lat.set_populations(f0.reshape(-1))
 
@@ -89,7 +102,7 @@ def test_noalloc_matches_lattice_entry_point(q, storage):
     desc.periodic[0] = desc.periodic[1] = desc.periodic[2] = 1
     desc.storage = _abi.STORAGE[storage]
     desc.device = 0
-    bulk = ob.BGKdynamics(omega=omega).params()
+    bulk = dynamics.params()
 
     desc_q = ob.descriptor(q)
 
@@ -108,22 +121,23 @@ def test_noalloc_matches_lattice_entry_point(q, storage):
     steps_done = 0
     try:
         for call, steps in enumerate((3, 3)):  # two calls in a row; the second starts at odd parity
-            ref_stats = lat.collide_and_stream(steps, stats=True)
+            ref_stats = lat.collide_and_stream(steps, stats=stats)
             ref_pops = lat.get_populations().reshape(q, -1).astype(np.float64)
 
             st = _abi.Stats()
             rc = lib.olb_b200_collide_and_stream_noalloc(ctypes.byref(desc), ctypes.c_void_p(buf.data_ptr()),
                                                         steps_done, ctypes.byref(bulk), steps,
-                                                        ctypes.byref(st), None)
+                                                        ctypes.byref(st) if stats else None, None)
             _abi.check(lib, rc)
             steps_done += steps
             torch.cuda.synchronize()
 
             # statistics of the last step
-            for key in ("sum_rho", "sum_usqr", "max_usqr", "average_rho", "average_energy", "max_u"):
+            for key in () if not stats else ("sum_rho", "sum_usqr", "max_usqr", "average_rho", "average_energy", "max_u"):
                 np.testing.assert_allclose(getattr(st, key), ref_stats[key], rtol=RTOL_STATS[key], err_msg=key)
-            assert st.n_cells == ref_stats["n_cells"] == n
-            assert st.n_nonfinite == 0
+            if stats:
+                assert st.n_cells == ref_stats["n_cells"] == n
+                assert st.n_nonfinite == 0
 
             # populations after each call
             got = logical(buf, steps_done)
