@@ -249,6 +249,10 @@ def descriptor(q: int):
 # --------------------------------------------------------------------------
 # the compiled reference (OpenLB CPU_SISD / CPU_SIMD through its public API)
 
+class ReferenceMissing(RuntimeError):
+    """A program built from OpenLB's sources is not there (tests are then skipped)."""
+
+
 def reference_binary(q: int, dtype, variant: str = "sisd") -> Path:
     bits = "f32" if np.dtype(dtype) == np.float32 else "f64"
     if variant == "simd":
@@ -258,6 +262,12 @@ def reference_binary(q: int, dtype, variant: str = "sisd") -> Path:
     if variant == "nocse":
         return REF_DIR / f"olb_ref_sisd_q{q}_{bits}_nocse"
     return REF_DIR / f"olb_ref_sisd_q{q}_{bits}"
+
+
+def _built(binary: Path) -> Path:
+    if not binary.exists():
+        raise ReferenceMissing(f"reference build missing: {binary} (make -C oracle/ref)")
+    return binary
 
 
 def write_case(dirpath: Path, case: Case, steps: int, init: np.ndarray | None = None,
@@ -333,7 +343,7 @@ def reference_normals(materials: np.ndarray, periodic, boundary_materials, q: in
     m = np.ascontiguousarray(materials, dtype=np.int32)
     size = m.shape
     n = m.size
-    binary = reference_binary(q, np.float64)
+    binary = _built(reference_binary(q, np.float64))
     with tempfile.TemporaryDirectory() as d:
         dp = Path(d)
         m.tofile(dp / "materials.i32")
@@ -358,9 +368,7 @@ def run_reference(case: Case, steps: int, dtype, init: np.ndarray | None = None,
                   threads: int | None = None, normals: bool = False,
                   load_checkpoint: bytes | None = None, save_checkpoint: bool = False):
     """Run OpenLB itself; returns dict(pops, rho, u[, stats][, checkpoint])."""
-    binary = reference_binary(case.q, dtype, variant)
-    if not binary.exists():
-        raise RuntimeError(f"reference build missing: {binary} (make -C oracle/ref)")
+    binary = _built(reference_binary(case.q, dtype, variant))
     with tempfile.TemporaryDirectory() as d:
         write_case(Path(d), case, steps, init=init, rhou=rhou, stats=stats, normals=normals,
                    load_checkpoint=load_checkpoint, save_checkpoint=save_checkpoint)

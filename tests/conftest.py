@@ -13,6 +13,15 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "reference: needs the compiled reference build in oracle/_ref")
 
 
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_call(item):
+    """Tests that run OpenLB's own programs are skipped where those are not built."""
+    outcome = yield
+    from oracle.oracle import ReferenceMissing
+    if outcome.excinfo is not None and issubclass(outcome.excinfo[0], ReferenceMissing):
+        outcome.force_exception(pytest.skip.Exception(str(outcome.excinfo[1])))
+
+
 @pytest.fixture(scope="session")
 def oracle_mod():
     from oracle import oracle as O

@@ -28,6 +28,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+from oracle.oracle import ReferenceMissing
 from tests.olb_vtk import read_vti
 
 pytestmark = pytest.mark.gpu
@@ -38,7 +39,8 @@ SIZE, STEPS = 32, 100   # the example runs 10 warm-up steps before STEPS timed o
 
 def _run(binary: str, workdir: Path, *args, env=None):
     exe = BIN / binary
-    assert exe.exists(), f"{exe} missing: build it with make -C openlb_b200/platform"
+    if not exe.exists():
+        raise ReferenceMissing(f"{exe} missing: build it with make -C openlb_b200/platform")
     r = subprocess.run([str(exe), *map(str, args)], cwd=workdir, capture_output=True, text=True,
                        timeout=600, env=dict(os.environ, **(env or {})))
     assert r.returncode == 0, f"{binary} failed ({r.returncode}): {r.stdout[-1500:]} {r.stderr[-1500:]}"
