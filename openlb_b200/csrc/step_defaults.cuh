@@ -18,21 +18,31 @@ namespace olb_b200 {
 //   16-bit: D3Q19's two-lane collision fits the 64 registers of {1,4}; D3Q27's
 // needs the 80 of {1,3} (160^3 masked BF16 81.6 against 92.9).
 //   FP64: {1,3} (160^3 D3Q19 masked 189 against 191 {1,4}; D3Q27 128^3 140 against
-// 164 {1,4} and 146 {2,2}).
+// 164 {1,4} and 146 {2,2}), but the forced D3Q27 collisions, whose registers spill
+// under the cap of {1,3}, take {2,2} above one wave (forced TRT with walls 64^3 20.9
+// against 29.8, 128^3 182 against 243, 160^3 338 against 463; open 128^3 158 against
+// 172; in one wave, 36^3 open, 9.1 against 6.6).
 //   FP32: {1,4} (64^3 open 5.80 against 6.49 {2,3}, 256^3 open forced TRT 417
 // against 430), but two cells per thread {2,3} where they win: from 2^21 cells
 // open boxes without a force (256^3 389 against 393, 160^3 100.0 against 99.4 but
-// 3 % less with statistics every step, 96^3 16.2 against 15.9) and masked
+// 3 % less with statistics every step, 96^3 16.2 against 15.9) and masked D3Q19
 // lattices with one (200^3 207 against 214, 128^3 57.4 against 58.4, 96^3 20.2
-// against 19.6).
+// against 19.6; not D3Q27: 144^3 117 against 109, 128^3 84.7 against 78.2).
+//   The bound of one wave is that of the collisions without a force; 16-bit D3Q19
+// forced TRT would still gain from {1,3} at 64^3 (5.45 against 6.00) and 80^3 (8.96
+// against 9.24).
+constexpr size_t kSMs = 148;  // of a B200
+
+inline bool is_forced(int kind) { return kind == K_FORCED_BGK || kind == K_FORCED_TRT; }
+
 inline int default_step_variant(int q, int bytes, bool masked, int kind, size_t cells)
 {
-  constexpr size_t kOneWave = size_t(148) * 3 * kStepThreads;
-  const bool one_wave = (bytes == 2 ? (cells + 1) / 2 : cells) <= kOneWave;
-  if (bytes == 8 || one_wave) return 0;
+  const bool one_wave = (bytes == 2 ? (cells + 1) / 2 : cells) <= kSMs * 3 * kStepThreads;
+  if (one_wave) return 0;
+  if (bytes == 8) return q == 27 && is_forced(kind) ? 2 : 0;
   if (bytes == 2) return q == 27 ? 0 : 1;
-  const bool forced = kind == K_FORCED_BGK || kind == K_FORCED_TRT;
-  return forced == masked && cells >= size_t(1) << 21 ? 3 : 1;
+  const bool two_cells = is_forced(kind) ? masked && q == 19 : !masked;
+  return two_cells && cells >= size_t(1) << 21 ? 3 : 1;
 }
 
 } // namespace olb_b200

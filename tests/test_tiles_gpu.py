@@ -270,6 +270,26 @@ def test_tuning_reports_the_kernel_that_runs(storage, nx, kernels):
         assert lat.autotune(2)["candidates"] == 3 * len(set(kernels))
 
 
+# the default of each lattice class on both sides of its changes: one wave (148 * 3
+# blocks of 256 threads: 48 x 48 x 49 cells fit, 49 x 51 x 47 do not), 2^21 cells
+@pytest.mark.parametrize("q,storage,size,open_,walls,open_forced,walls_forced", [
+    (19, "f32", (48, 48, 49), 0, 0, 0, 0), (19, "f32", (49, 51, 47), 1, 1, 1, 1), (19, "f32", (128, 128, 128), 3, 1, 1, 3),
+    (27, "f32", (49, 51, 47), 1, 1, 1, 1), (27, "f32", (128, 128, 128), 3, 1, 1, 1),
+    (19, "f64", (49, 51, 47), 0, 0, 0, 0), (27, "f64", (48, 48, 49), 0, 0, 0, 0), (27, "f64", (49, 51, 47), 0, 0, 2, 2),
+    (19, "f16", (49, 51, 47), 0, 0, 0, 0), (19, "f16", (80, 80, 80), 1, 1, 1, 1), (27, "bf16", (80, 80, 80), 0, 0, 0, 0),
+])
+def test_default_step_variants(q, storage, size, open_, walls, open_forced, walls_forced):
+    n = size[0] * size[1] * size[2]
+    ids = (np.arange(n) % 7 == 0).astype(np.uint8)
+    got = []
+    with ob.Lattice(q, size, (True,) * 3, storage=storage) as lat:
+        for bulk in (ob.BGKdynamics(omega=1.3), ob.ForcedTRTdynamics(omega=1.3, force=(1e-5, 0, 0))):
+            for table, cells in (([bulk], None), ([bulk, ob.BounceBack()], ids)):
+                lat.set_dynamics(table, cells)
+                got.append(lat.tuning()["variant"])
+    assert got == [open_, walls, open_forced, walls_forced]
+
+
 @pytest.mark.parametrize("drop", ["set_dynamics", "set_step_variant"])
 def test_a_dropped_tuning_takes_its_launch_shape_along(drop):
     """What the autotuner chose for one kernel class is not left to another: the lattice
