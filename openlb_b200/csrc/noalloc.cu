@@ -158,6 +158,7 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   set_flat(g, kStepThreads);
   const dim3 stat_grid = step_grid(g, bz, by, step_cells(g, elem, variant));
   blocks = size_t(stat_grid.x) * stat_grid.y * stat_grid.z;
+  const bool chain = chain_steps(desc->q, elem, bulk->kind, blocks);
 
   cudaError_t e = cudaSetDevice(desc->device);
   if (e != cudaSuccess) return noalloc_cuda(e, "cudaSetDevice");
@@ -184,7 +185,7 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
     a.table = nullptr;
     a.bulk = params;
     if (last_stats) a.sink.partials = scratch->partials;
-    a.chained = k > 0;  // what the caller enqueued before is not overlapped
+    a.chained = k > 0 && chain;  // what the caller enqueued before is not overlapped
     a.block_z = bz;
     a.block_y = by;
     a.variant = variant;

@@ -571,6 +571,7 @@ olb_b200_status boundary_noise(olb_b200_lattice* L);
 
 olb_b200_status enqueue_steps(olb_b200_lattice* L, int steps, bool stats_last)
 {
+  const bool chain = chain_steps(L->q, int(L->elem), L->bulk_kind, step_blocks(L));
   for (int s = 0; s < steps; ++s) {
     olb_b200_status nst = boundary_noise(L);
     if (nst != OLB_B200_OK) return nst;
@@ -582,7 +583,7 @@ olb_b200_status enqueue_steps(olb_b200_lattice* L, int steps, bool stats_last)
     a.table = L->table;
     a.bulk = L->bulk;
     if (stats) a.sink = stat_sink(L, step_blocks(L), L->n_bc == 0);
-    a.chained = true;
+    a.chained = chain;
     a.block_z = L->block_z;
     a.block_y = L->block_y;
     a.variant = L->variant;

@@ -1,4 +1,5 @@
-// Which step kernel a lattice takes unless told otherwise.
+// Which step kernel a lattice takes unless told otherwise, and how its steps are
+// launched.
 #pragma once
 
 #include <cstddef>
@@ -43,6 +44,20 @@ inline int default_step_variant(int q, int bytes, bool masked, int kind, size_t 
   if (bytes == 2) return q == 27 ? 0 : 1;
   const bool two_cells = is_forced(kind) ? masked && q == 19 : !masked;
   return two_cells && cells >= size_t(1) << 21 ? 3 : 1;
+}
+
+// Whether a step of `blocks` blocks may start before the one ahead of it has ended
+// (launch_chained).  It hides a launch of 4 to 6 us; but a grid that leaves SMs
+// empty then shares SMs with its predecessor, and where a block keeps the FP64 pipe
+// of its SM busy by itself, the two take turns: D3Q27 FP64 forced TRT 24^3 (72
+// blocks) 6.8 us chained against 6.2, 32^3 (128) 8.3 against 6.2, with walls 10.0
+// against 7.7.  With at most 64 blocks two grids fit side by side (20^3 5.8 against
+// 6.2), above one block per SM both share anyway (36^3, 216 blocks, 6.6 against
+// 8.3).  The collisions without a force gain or are even (28^3 5.2 against 5.6; the
+// worst, 32^3 Smagorinsky with walls, 7.3 against 6.2).
+inline bool chain_steps(int q, int bytes, int kind, size_t blocks)
+{
+  return !(bytes == 8 && q == 27 && is_forced(kind) && blocks > 64 && blocks <= kSMs);
 }
 
 } // namespace olb_b200
