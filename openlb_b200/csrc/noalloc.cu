@@ -214,7 +214,7 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   if (!stats) return OLB_B200_OK;
 
   // one block: no counter that calls overlapping by mistake could leave behind
-  e = launch_chained(reduce_partials_kernel, false, dim3(1), dim3(1024), s, scratch->partials, blocks, nullptr,
+  e = launch_chained(reduce_partials_kernel, true, dim3(1), dim3(1024), s, scratch->partials, blocks, nullptr,
                      &scratch->result, 0ull);
   if (e != cudaSuccess) return noalloc_cuda(e, "statistics reduction launch");
   StatPartial p;
