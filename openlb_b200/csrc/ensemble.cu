@@ -543,11 +543,17 @@ olb_b200_status upload_tables(olb_b200_ensemble* E)
 
 olb_b200_status enqueue_chunk(olb_b200_ensemble* E, int steps, int check)
 {
+  // A chained step shares SMs with the one ahead of it, unless two grids fit side by
+  // side (64 blocks).  Where all tiles fit the SMs at once that can cost more than the
+  // launch it hides: 50 steps of one 32^3 cavity (128 tiles) 177 us in order, 218
+  // chained, 40^3 (250) 204 and 239, 48^3 (432) 242 and 287; but 36^3 (183) 226 and
+  // 203.  Of 20^3 (32) 201 and 189, of four of 24..48 (1242) 499 and 485.
+  const bool chain = E->step_grid <= 64 || E->step_grid > 148 * E->min_blocks;
   for (int k = 0; k < steps; ++k) {
     const auto kernel = E->min_blocks == 2   ? ensemble_step_kernel<2>
                         : E->min_blocks == 4 ? ensemble_step_kernel<4>
                                              : ensemble_step_kernel<3>;
-    OLB_ECUDA(launch_chained(kernel, k > 0, dim3(unsigned(E->step_grid)), dim3(kEnsembleThreads), E->stream, E->pool,
+    OLB_ECUDA(launch_chained(kernel, chain && k > 0, dim3(unsigned(E->step_grid)), dim3(kEnsembleThreads), E->stream, E->pool,
                              E->table_dev, E->tiles_dev, E->ntiles_dev, k));
   }
   if (check) {
