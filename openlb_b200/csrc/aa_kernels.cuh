@@ -322,9 +322,10 @@ constexpr StepVariant kStepVariants[] = {{1, 3}, {1, 4}, {2, 2}, {2, 3}};
 #endif
 constexpr int kNumStepVariants = 4;
 
-// 16-bit storage in the natural layout (one cell per element) takes two cells
-// per thread as the lanes of the packed collision (aa_step_split_kernel); the
-// reference-order build collides one cell at a time
+// 16-bit storage in the natural layout (one cell per element) has two kernels:
+// one cell per thread (variants 0 and 2), and two as the lanes of the packed
+// collision (variants 1 and 3, aa_step_split_kernel).  The reference-order build
+// collides one cell at a time.
 #ifdef OLB_B200_EXACT
 constexpr bool kSplitNatural16 = false;
 #else
@@ -341,6 +342,9 @@ constexpr StepVariant step_variant(int bytes, int v)
 {
   return kStepVariants[bytes == 2 ? v & 1 : v];
 }
+
+// whether a natural 16-bit lattice runs aa_step_split_kernel in variant v
+constexpr bool split_variant(int v) { return kSplitNatural16 && (v & 1) != 0; }
 
 // running sums of the fused statistics of one thread
 struct StatAcc {
@@ -1853,10 +1857,13 @@ inline dim3 step_grid(const Geometry& g, int bz, int by, int cells_per_thread)
 // FP32 gains nothing from it (257^3 cavity 418 against 417 us with 128).
 inline int flat_threads(int bytes) { return bytes == 2 ? 64 : kStepThreads; }
 
-// Cells per thread of the step kernel that serves a lattice.
-inline int step_cells(const Geometry& g, int bytes, int variant)
+// What runs on a lattice when variant v is selected.
+inline StepVariant running_variant(const Geometry& g, int bytes, int v)
 {
-  return bytes == 2 && !g.paired && kSplitNatural16 ? 2 : step_variant(bytes, variant).cells_per_thread;
+  if (bytes == 2 && !g.paired && kSplitNatural16) {
+    return split_variant(v) ? StepVariant{2, kSplitMinBlocks} : kStepVariants[0];
+  }
+  return step_variant(bytes, v);
 }
 
 inline dim3 step_block(const Geometry& g, int bz, int by)

@@ -14,7 +14,8 @@ template <int Q, class S, class R, int KIND, int CPT, int MINB, bool ODD, bool S
 static cudaError_t launch_step_one(const StepLaunch& a, bool masked)
 {
   const dim3 block = step_block(a.g, a.block_z, a.block_y);
-  const dim3 grid = step_grid(a.g, a.block_z, a.block_y, step_cells(a.g, int(sizeof(S)), a.variant));
+  const dim3 grid =
+    step_grid(a.g, a.block_z, a.block_y, running_variant(a.g, int(sizeof(S)), a.variant).cells_per_thread);
   S* pops = static_cast<S*>(a.pops);
   const DynDevice<R>* table = static_cast<const DynDevice<R>*>(a.table);
   const DynDevice<R>& bulk = *static_cast<const DynDevice<R>*>(a.bulk);
@@ -27,19 +28,20 @@ static cudaError_t launch_step_one(const StepLaunch& a, bool masked)
                                      a.stream, pops, a.g, bulk, a.sink);
     }
     if constexpr (kSplitNatural16) {
-      return masked ? launch_chained(aa_step_split_kernel<Q, S, KIND, ODD, true, STATS>, a.chained, grid, block,
-                                     a.stream, pops, a.g, a.ids, table, bulk, a.sink)
-                    : launch_chained(aa_step_split_kernel<Q, S, KIND, ODD, false, STATS>, a.chained, grid, block,
-                                     a.stream, pops, a.g, a.ids, table, bulk, a.sink);
+      if (split_variant(a.variant)) {
+        return masked ? launch_chained(aa_step_split_kernel<Q, S, KIND, ODD, true, STATS>, a.chained, grid, block,
+                                       a.stream, pops, a.g, a.ids, table, bulk, a.sink)
+                      : launch_chained(aa_step_split_kernel<Q, S, KIND, ODD, false, STATS>, a.chained, grid, block,
+                                       a.stream, pops, a.g, a.ids, table, bulk, a.sink);
+      }
     }
   }
-  if constexpr (!kHalf || !kSplitNatural16) {
-    return masked ? launch_chained(aa_step_masked_kernel<Q, S, R, KIND, ODD, STATS, CPT, MINB>, a.chained, grid, block,
-                                   a.stream, pops, a.g, a.ids, table, bulk, a.sink)
-                  : launch_chained(aa_step_kernel<Q, S, R, KIND, ODD, STATS, CPT, MINB>, a.chained, grid, block,
-                                   a.stream, pops, a.g, bulk, a.sink);
-  }
-  return cudaErrorInvalidValue;
+  // the natural 16-bit layout compiles one variant of the one-cell kernels
+  constexpr StepVariant one = kHalf && kSplitNatural16 ? kStepVariants[0] : StepVariant{CPT, MINB};
+  return masked ? launch_chained(aa_step_masked_kernel<Q, S, R, KIND, ODD, STATS, one.cells_per_thread, one.min_blocks>,
+                                 a.chained, grid, block, a.stream, pops, a.g, a.ids, table, bulk, a.sink)
+                : launch_chained(aa_step_kernel<Q, S, R, KIND, ODD, STATS, one.cells_per_thread, one.min_blocks>,
+                                 a.chained, grid, block, a.stream, pops, a.g, bulk, a.sink);
 }
 
 template <int Q, class S, class R, int KIND, int CPT, int MINB>

@@ -154,9 +154,9 @@ extern "C" olb_b200_status olb_b200_collide_and_stream_noalloc(
   // per step with two cells per thread, 432 with one).  Flat tiles of
   // kStepThreads, which a step with statistics takes, need no more blocks than
   // the limit counts.
-  const int variant = default_step_variant(desc->q, elem, false, bulk->kind, cells);
+  const int variant = default_step_variant(desc->q, elem, false, false, bulk->kind, cells);
   set_flat(g, kStepThreads);
-  const dim3 stat_grid = step_grid(g, bz, by, step_cells(g, elem, variant));
+  const dim3 stat_grid = step_grid(g, bz, by, running_variant(g, elem, variant).cells_per_thread);
   blocks = size_t(stat_grid.x) * stat_grid.y * stat_grid.z;
   const bool chain = chain_steps(desc->q, elem, bulk->kind, blocks);
 

@@ -332,19 +332,12 @@ void default_shape(const olb_b200_lattice* L, int& bz, int& by)
 
 int default_variant(const olb_b200_lattice* L)
 {
-  return default_step_variant(L->q, int(L->elem), L->masked, L->bulk_kind, L->cells);
+  return default_step_variant(L->q, int(L->elem), L->g.paired != 0, L->masked, L->bulk_kind, L->cells);
 }
 
 int cells_per_thread(const olb_b200_lattice* L)
 {
-  return step_cells(L->g, int(L->elem), L->variant);
-}
-
-// What runs when variant v is selected: the natural 16-bit layout has one kernel
-StepVariant running_variant(const olb_b200_lattice* L, int v)
-{
-  if (L->elem == 2 && !L->g.paired && kSplitNatural16) return StepVariant{2, kSplitMinBlocks};
-  return step_variant(int(L->elem), v);
+  return running_variant(L->g, int(L->elem), L->variant).cells_per_thread;
 }
 
 // How the step kernels cut a plane: flat tiles (flat_threads) unless a launch
@@ -1418,7 +1411,7 @@ olb_b200_status olb_b200_get_tuning(olb_b200_lattice* L, olb_b200_tuning* out)
 {
   if (!L || !out) return fail(OLB_B200_ERR_ARG, "get_tuning: null argument");
   out->variant = L->variant;
-  const StepVariant running = running_variant(L, L->variant);
+  const StepVariant running = running_variant(L->g, int(L->elem), L->variant);
   out->cells_per_thread = running.cells_per_thread;
   out->min_blocks_per_sm = running.min_blocks;
   const dim3 block = step_block(L->g, L->block_z, L->block_y);
@@ -1457,7 +1450,7 @@ olb_b200_status olb_b200_autotune(olb_b200_lattice* L, int32_t trial_steps, olb_
   for (int v = 0; v < kNumStepVariants && st == OLB_B200_OK; ++v) {
     bool duplicate = false;
     for (int w = 0; w < v; ++w) {
-      const StepVariant a = running_variant(L, v), b = running_variant(L, w);
+      const StepVariant a = running_variant(L->g, int(L->elem), v), b = running_variant(L->g, int(L->elem), w);
       duplicate |= a.cells_per_thread == b.cells_per_thread && a.min_blocks == b.min_blocks;
     }
     if (duplicate) continue;

@@ -18,6 +18,12 @@ namespace olb_b200 {
 // thread: FP16 60^3 3.80 against 4.36, 64^3 4.43 against 4.23.
 //   16-bit: D3Q19's two-lane collision fits the 64 registers of {1,4}; D3Q27's
 // needs the 80 of {1,3} (160^3 masked BF16 81.6 against 92.9).
+//   16-bit, natural layout: two cells per thread (variant 1), but one (variant 0)
+// where the lattice leaves lanes to spare and the longer thread shows: D3Q27 up to
+// three blocks per SM (forced TRT with walls 33x32x32 4.3 against 7.0, 49x48x48 4.9
+// against 7.3; open BGK 33x32x32 4.1 against 5.4, 49x48x48 4.45 against 4.47, 61x60x60
+// 7.3 against 6.3), D3Q19 up to two (BGK with walls 41x40x40 3.6 against 4.1; open
+// 41x40x40 3.3 against 3.4, 49x48x48 4.2 against 3.4).
 //   FP64: {1,3} (160^3 D3Q19 masked 189 against 191 {1,4}; D3Q27 128^3 140 against
 // 164 {1,4} and 146 {2,2}), but the forced D3Q27 collisions, whose registers spill
 // under the cap of {1,3}, take {2,2} above one wave (forced TRT with walls 64^3 20.9
@@ -36,9 +42,10 @@ constexpr size_t kSMs = 148;  // of a B200
 
 inline bool is_forced(int kind) { return kind == K_FORCED_BGK || kind == K_FORCED_TRT; }
 
-inline int default_step_variant(int q, int bytes, bool masked, int kind, size_t cells)
+inline int default_step_variant(int q, int bytes, bool paired, bool masked, int kind, size_t cells)
 {
-  const bool one_wave = (bytes == 2 ? (cells + 1) / 2 : cells) <= kSMs * 3 * kStepThreads;
+  if (bytes == 2 && !paired) return cells <= kSMs * (q == 27 ? 3 : 2) * kStepThreads ? 0 : 1;
+  const bool one_wave = (paired ? (cells + 1) / 2 : cells) <= kSMs * 3 * kStepThreads;
   if (one_wave) return 0;
   if (bytes == 8) return q == 27 && is_forced(kind) ? 2 : 0;
   if (bytes == 2) return q == 27 ? 0 : 1;

@@ -21,11 +21,13 @@ STEPS = 4
 UNIT = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8}
 
 
-def advance(case, f0, steps, storage, shape=None):
+def advance(case, f0, steps, storage, shape=None, variant=None):
     with ob.Lattice(case.q, case.size, case.periodic, storage=storage) as lat:
         lat.set_dynamics(C.to_abi_table(case), case.dyn_id)
         if shape:
             lat.set_launch_shape(*shape)
+        if variant is not None:
+            lat.set_step_variant(variant)
         lat.set_populations(f0)
         lat.collide_and_stream(steps)
         return lat.get_populations()
@@ -47,13 +49,15 @@ def check(case, f0, got, storage):
 PLANES = [(1, 1), (7, 9), (4, 16), (5, 13), (8, 16), (3, 43), (5, 51), (16, 16), (257, 1), (19, 27)]
 
 
-@pytest.mark.parametrize("storage,nx", [("f32", 3), ("f16", 4), ("f16", 3), ("bf16", 5)])
+# 16-bit with odd nx: one cell per thread (variant 0) and two (1)
+@pytest.mark.parametrize("storage,nx,variant", [("f32", 3, None), ("f16", 4, None), ("f16", 3, 0), ("f16", 3, 1),
+                                                ("bf16", 5, 0), ("bf16", 5, 1)])
 @pytest.mark.parametrize("plane", PLANES)
-def test_periodic_planes_around_a_block(storage, nx, plane):
+def test_periodic_planes_around_a_block(storage, nx, variant, plane):
     rng = np.random.default_rng(31 + plane[0])
     case = C.periodic_case(19, (nx,) + plane, kind=O.FORCED_TRT)
     f0 = C.random_state(19, case.n, np.float32, rng)
-    check(case, f0, advance(case, f0, STEPS, storage), storage)
+    check(case, f0, advance(case, f0, STEPS, storage, variant=variant), storage)
 
 
 @pytest.mark.parametrize("storage", ["f32", "f64"])
@@ -76,14 +80,15 @@ def test_planes_around_a_block_in_every_step_variant(storage, variant, plane):
     assert rel <= rtol, rel
 
 
-@pytest.mark.parametrize("q,storage,nx", [(19, "f16", 5), (27, "bf16", 5), (19, "f16", 6), (19, "f32", 5)])
+@pytest.mark.parametrize("q,storage,nx,variant", [(19, "f16", 5, 0), (19, "f16", 5, 1), (27, "bf16", 5, 0),
+                                                  (27, "bf16", 5, 1), (19, "f16", 6, None), (19, "f32", 5, None)])
 @pytest.mark.parametrize("plane", [(7, 9), (3, 43), (16, 16), (9, 57)])
-def test_cavity_planes_around_a_block(q, storage, nx, plane):
+def test_cavity_planes_around_a_block(q, storage, nx, variant, plane):
     rng = np.random.default_rng(57 + plane[1])
     case = C.cavity_case(q, (nx,) + plane)
     f0 = C.random_state(q, case.n, np.float32, rng, amp_u=0.01)
     # slots fed from outside the box hold what the wrap brings; only walls read them
-    check(case, f0, advance(case, f0, STEPS, storage), storage)
+    check(case, f0, advance(case, f0, STEPS, storage, variant=variant), storage)
 
 
 def test_flat_tiles_and_rectangles_agree():
@@ -201,11 +206,12 @@ def test_force_field_outlives_set_dynamics():
 
 
 @pytest.mark.parametrize("q,storage", [(19, "f16"), (19, "bf16"), (27, "f16")])
+@pytest.mark.parametrize("variant", [0, 1])
 @pytest.mark.parametrize("kind", [ob.BGKdynamics(omega=1.2), ob.ForcedBGKdynamics(omega=1.2, force=(1e-4, 0, 0))],
                          ids=["bgk", "forced"])
-def test_cells_that_pass_through_keep_their_bits(q, storage, kind):
-    """NoDynamics cells among fluid, walls and moving walls in 16-bit storage, odd nx: what
-    streams out of them is what was stored, bit for bit, with pairs of populations of
+def test_cells_that_pass_through_keep_their_bits(q, storage, kind, variant):
+    """NoDynamics cells among fluid, walls and moving walls in 16-bit storage, odd nx (one
+    cell per thread and two): what streams out of them is what was stored, bit for bit, with pairs of populations of
     very different size and with an infinity or NaN in one population of a cell."""
     rng = np.random.default_rng(5)
     size = (5, 9, 29)
@@ -218,6 +224,7 @@ def test_cells_that_pass_through_keep_their_bits(q, storage, kind):
     source = (ids == 1).reshape(size)
     with ob.Lattice(q, size, (True,) * 3, storage=storage) as lat:
         lat.set_dynamics([kind, ob.NoDynamics(), ob.BounceBack(), ob.BounceBackVelocity((0.03, 0, 0))], ids)
+        lat.set_step_variant(variant)
         lat.set_populations(f0.reshape(-1))
         before = lat.get_populations().reshape((q,) + size)
         for _ in range(3):  # both parities
@@ -256,7 +263,7 @@ def test_a_launch_shape_is_what_runs(storage, nx):
 
 # launch shapes timed at nz = 75: 64x4, 32x8 and flat tiles
 @pytest.mark.parametrize("storage,nx,kernels", [
-    ("f16", 5, [(2, 3)] * 4),                              # the natural layout's one kernel
+    ("f16", 5, [(1, 3), (2, 3), (1, 3), (2, 3)]),          # natural layout: one or two cells
     ("f16", 6, [(1, 3), (1, 4), (1, 3), (1, 4)]),          # one element per thread
     ("f32", 5, [(1, 3), (1, 4), (2, 2), (2, 3)]),
 ])
@@ -276,7 +283,10 @@ def test_tuning_reports_the_kernel_that_runs(storage, nx, kernels):
     (19, "f32", (48, 48, 49), 0, 0, 0, 0), (19, "f32", (49, 51, 47), 1, 1, 1, 1), (19, "f32", (128, 128, 128), 3, 1, 1, 3),
     (27, "f32", (49, 51, 47), 1, 1, 1, 1), (27, "f32", (128, 128, 128), 3, 1, 1, 1),
     (19, "f64", (49, 51, 47), 0, 0, 0, 0), (27, "f64", (48, 48, 49), 0, 0, 0, 0), (27, "f64", (49, 51, 47), 0, 0, 2, 2),
-    (19, "f16", (49, 51, 47), 0, 0, 0, 0), (19, "f16", (80, 80, 80), 1, 1, 1, 1), (27, "bf16", (80, 80, 80), 0, 0, 0, 0),
+    (19, "f16", (48, 64, 64), 0, 0, 0, 0), (19, "f16", (80, 80, 80), 1, 1, 1, 1), (27, "bf16", (80, 80, 80), 0, 0, 0, 0),
+    # natural 16-bit layout: two blocks per SM (75 776 cells) in D3Q19, three in D3Q27
+    (19, "f16", (37, 64, 32), 0, 0, 0, 0), (19, "bf16", (37, 64, 33), 1, 1, 1, 1),
+    (27, "bf16", (37, 64, 48), 0, 0, 0, 0), (27, "f16", (49, 51, 47), 1, 1, 1, 1),
 ])
 def test_default_step_variants(q, storage, size, open_, walls, open_forced, walls_forced):
     n = size[0] * size[1] * size[2]

@@ -58,8 +58,8 @@ BGK, FORCED_TRT = ob.BGKdynamics(omega=1.3), ob.ForcedTRTdynamics(omega=1.3, for
 # odd nx: a 16-bit handle then keeps one cell per element, the layout the
 # no-allocation call takes.  FP32 takes {1,3} up to one wave of 148 * 3 * 256 =
 # 113 664 cells, {1,4} above, and {2,3} from 2^21 cells on without a force; FP64
-# {1,3}, or {2,2} above one wave for forced D3Q27; 16-bit storage the two-cell
-# kernel of the natural layout.
+# {1,3}, or {2,2} above one wave for forced D3Q27; 16-bit storage one cell per
+# thread up to a wave (two blocks per SM in D3Q19), two above.
 SMALL, ABOVE_ONE_WAVE, LARGE = (41, 36, 70), (49, 51, 47), (129, 127, 131)
 
 
@@ -68,6 +68,7 @@ SMALL, ABOVE_ONE_WAVE, LARGE = (41, 36, 70), (49, 51, 47), (129, 127, 131)
     (27, "f16", SMALL, BGK, True),
     (19, "f32", ABOVE_ONE_WAVE, BGK, True), (19, "f32", ABOVE_ONE_WAVE, FORCED_TRT, True),
     (19, "f32", ABOVE_ONE_WAVE, BGK, False),
+    (27, "f16", ABOVE_ONE_WAVE, BGK, True), (19, "f16", (41, 36, 50), FORCED_TRT, True),
     (19, "f32", LARGE, BGK, True), (19, "f32", LARGE, BGK, False), (19, "f32", LARGE, FORCED_TRT, True),
     (27, "f64", ABOVE_ONE_WAVE, FORCED_TRT, True), (27, "f64", (28, 28, 28), FORCED_TRT, True),
     (27, "f32", LARGE, BGK, True), (19, "f64", LARGE, BGK, True), (19, "f16", LARGE, FORCED_TRT, False),
