@@ -21,9 +21,11 @@
  *     the last stream.  The element type is the compute type: double for
  *     OLB_B200_STORAGE_F64, float otherwise.  How the library keeps them in
  *     device memory (AA pattern, 16-bit storage) is internal.
- *   - Host pointers are borrowed for the duration of the call.  Results copied
- *     into memory that is not pinned pass through pinned buffers that all
- *     handles of a process share (8 MiB, given back with the last handle).  Device
+ *   - Host pointers are borrowed for the duration of the call.  Once the handles
+ *     of a process have copied 32 MiB of results into memory that is not pinned,
+ *     such copies of 1 MiB and more pass through pinned buffers that all handles
+ *     share (8 MiB) and are written by up to six threads, which sleep between
+ *     copies; both are given back with the last handle.  Device
  *     memory, the CUDA stream and any CUDA graphs are owned by the handle.
  *   - One host thread drives one lattice handle; distinct handles may be used
  *     from distinct threads.  All device work of a handle is ordered on its
@@ -285,7 +287,7 @@ olb_b200_status olb_b200_set_launch_shape(olb_b200_lattice* lattice, int32_t blo
  * only in speed; it picks a default per lattice class.  The reference has no
  * counterpart (its kernels launch 32-thread blocks, gpu/cuda/operator.hh:424-427). */
 typedef struct {
-  int32_t variant;            /* index of the step-kernel variant */
+  int32_t variant;            /* index of the step-kernel variant (0..3) */
   int32_t cells_per_thread;
   int32_t min_blocks_per_sm;  /* register cap = 65536 / (256 * min_blocks_per_sm) */
   int32_t block_z, block_y;
@@ -300,7 +302,9 @@ typedef struct {
  * not advance.  Synchronous. */
 olb_b200_status olb_b200_autotune(olb_b200_lattice* lattice, int32_t trial_steps, olb_b200_tuning* out);
 olb_b200_status olb_b200_get_tuning(olb_b200_lattice* lattice, olb_b200_tuning* out);
-/* Selects a variant explicitly (-1: the library's default for this lattice). */
+/* Selects a variant explicitly (-1: the library's default for this lattice).
+ * 16-bit lattices compile two: variants 2 and 3 are 0 and 1 there, and
+ * olb_b200_get_tuning gives what they run. */
 olb_b200_status olb_b200_set_step_variant(olb_b200_lattice* lattice, int32_t variant);
 
 /* Collide-and-stream on caller-owned device memory, allocating nothing.  This

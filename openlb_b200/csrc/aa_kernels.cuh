@@ -617,8 +617,8 @@ template <> struct Pair<__nv_bfloat16> {
 
 // what a lane of the two-lane collision does: collide with the lattice's fluid
 // kind, bounce back (full-way, collision::Revert), or pass its populations
-// through unchanged (NoDynamics, and boundary cells, whose collision ran ahead
-// of the step kernel)
+// through (NoDynamics, and boundary cells, whose collision ran ahead of the step
+// kernel), both up to an FP32 rounding of each pair's sum and difference
 enum LaneMode { kLaneFluid = 0, kLaneWall = 1, kLanePass = 2 };
 
 // the fluid collision constants of a cell for the scaled collisions (KIND the
@@ -1791,7 +1791,7 @@ struct StepLaunch {
   StatSink sink;           // partials: gridDim product entries (statistics only)
   bool chained = false;    // the previous work on the stream may be overlapped (launch_chained)
   int block_z, block_y;
-  int variant;             // index into kStepVariants
+  int variant;             // of the step kernel (running_variant)
   cudaStream_t stream;
 };
 
@@ -1871,14 +1871,19 @@ inline dim3 step_block(const Geometry& g, int bz, int by)
   return g.flat ? dim3(g.flat, 1) : dim3(bz, by);
 }
 
-// flat tiles of `threads` threads and the constants of their division by nz
+// the constants of floor(n / d) = (mulhi(n, mul) + n) >> shift for n < 2^31
+inline void division_constants(uint32_t d, uint32_t& mul, uint32_t& shift)
+{
+  shift = 0;
+  while ((uint64_t(1) << shift) < d) ++shift;
+  mul = uint32_t(((uint64_t(1) << 32) * ((uint64_t(1) << shift) - d)) / d + 1);
+}
+
+// flat tiles of `threads` threads
 inline void set_flat(Geometry& g, int threads)
 {
-  uint32_t s = 0;
-  while ((uint64_t(1) << s) < uint64_t(g.nz)) ++s;
   g.flat = threads;
-  g.flat_mul = uint32_t(((uint64_t(1) << 32) * ((uint64_t(1) << s) - uint64_t(g.nz))) / uint64_t(g.nz) + 1);
-  g.flat_shift = s;
+  division_constants(uint32_t(g.nz), g.flat_mul, g.flat_shift);
 }
 
 // grid of the gather / moments kernels (one cell per thread)

@@ -58,10 +58,9 @@ struct FastDiv {
   uint32_t s;
   static FastDiv make(uint32_t d)
   {
-    uint32_t s = 0;
-    while ((uint64_t(1) << s) < d) ++s;
-    const uint64_t m = ((uint64_t(1) << 32) * ((uint64_t(1) << s) - d)) / d + 1;
-    return FastDiv{uint32_t(m), s};
+    FastDiv f;
+    division_constants(d, f.m, f.s);
+    return f;
   }
   OLB_HD uint32_t div(uint32_t n) const
   {

@@ -61,10 +61,10 @@ using namespace olb_b200;
 namespace {
 
 // Scratch for the per-block statistics partials plus the reduced result:
-// 65536 * 40 B = 2.5 MiB per device.  A call with statistics
-// launches ceil(nz/bz) * ceil(ny/by) * nx blocks, (bz, by) = (128, 2) for
-// nz >= 128, (64, 4) for nz >= 64, else (32, 8): 65536 blocks cover a
-// 256 x 256 x 256 lattice, but only 2048 x 256 x 16 for a thin one.
+// 65536 * 40 B = 2.5 MiB per device.  A call with statistics is admitted when
+// ceil(nz/bz) * ceil(ny/by) * nx blocks fit, (bz, by) = (128, 2) for nz >= 128,
+// (64, 4) for nz >= 64, else (32, 8): a 256 x 256 x 256 lattice does, of thin ones
+// only 2048 x 256 x 16.  The flat tiles that it launches are no more than those.
 constexpr size_t kMaxBlocks = 65536;
 struct Scratch {
   StatPartial partials[kMaxBlocks];

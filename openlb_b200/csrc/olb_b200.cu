@@ -485,8 +485,9 @@ olb_b200_status ensure_partials(olb_b200_lattice* L)
 }
 
 // Blocks up to which the kernel that writes the partials also reduces them: its
-// last block then adds up at most four per thread, which is quicker than
-// another launch (32^3 cavity with statistics every step: 29.5 us a
+// last block then adds up at most four per thread where it has 256 (a launch shape
+// set by the caller may have fewer, down to 32), which is quicker than another
+// launch (32^3 cavity with statistics every step: 29.5 us a
 // step with reduction kernel, copy and synchronisation, 16.0 with this and
 // chained launches).  More go
 // through reduce_partials_kernel, one block per 1024.
