@@ -22,8 +22,9 @@ namespace olb_b200 {
 // where the lattice leaves lanes to spare and the longer thread shows: D3Q27 up to
 // three blocks per SM (forced TRT with walls 33x32x32 4.3 against 7.0, 49x48x48 4.9
 // against 7.3; open BGK 33x32x32 4.1 against 5.4, 49x48x48 4.45 against 4.47, 61x60x60
-// 7.3 against 6.3), D3Q19 up to two (BGK with walls 41x40x40 3.6 against 4.1; open
-// 41x40x40 3.3 against 3.4, 49x48x48 4.2 against 3.4).
+// 7.3 against 6.3), D3Q19 up to two (BGK with walls 41x40x40 3.6 against 4.1; open TRT
+// 33x32x32 2.9 against 4.0, 49x48x48 4.2 against 3.5), but not open BGK, the shortest
+// (36x34x21 caller-owned 2.8 against 2.6, 17^3 to 33^3 3.4 against 3.2).
 //   FP64: {1,3} (160^3 D3Q19 masked 189 against 191 {1,4}; D3Q27 128^3 140 against
 // 164 {1,4} and 146 {2,2}), but the forced D3Q27 collisions, whose registers spill
 // under the cap of {1,3}, take {2,2} above one wave (forced TRT with walls 64^3 20.9
@@ -44,7 +45,10 @@ inline bool is_forced(int kind) { return kind == K_FORCED_BGK || kind == K_FORCE
 
 inline int default_step_variant(int q, int bytes, bool paired, bool masked, int kind, size_t cells)
 {
-  if (bytes == 2 && !paired) return cells <= kSMs * (q == 27 ? 3 : 2) * kStepThreads ? 0 : 1;
+  if (bytes == 2 && !paired) {
+    const bool shortest = q == 19 && !masked && kind == K_BGK;
+    return !shortest && cells <= kSMs * (q == 27 ? 3 : 2) * kStepThreads ? 0 : 1;
+  }
   const bool one_wave = (paired ? (cells + 1) / 2 : cells) <= kSMs * 3 * kStepThreads;
   if (one_wave) return 0;
   if (bytes == 8) return q == 27 && is_forced(kind) ? 2 : 0;
