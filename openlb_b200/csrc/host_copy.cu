@@ -25,7 +25,7 @@
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
-#include <cstdlib>
+#include <cstdint>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -40,6 +40,7 @@ constexpr size_t kChunk = size_t(512) << 10;
 constexpr size_t kRing = 16;                     // 8 MiB of pinned memory per process
 constexpr size_t kStagedFrom = size_t(1) << 20;  // below, too few chunks to overlap
 constexpr size_t kHugePage = size_t(2) << 20;
+constexpr size_t kMapped = kRing * kChunk + kHugePage;
 // Making the ring and its threads and giving them back takes 1.5 ms (7 to 12 with
 // cudaHostAlloc, which pins 4 KiB pages), as much as staging saves on 10 MB of
 // fresh or 50 MB of reused memory.  They are made by the copy that brings what the
@@ -49,8 +50,10 @@ constexpr size_t kHugePage = size_t(2) << 20;
 constexpr size_t kRingFrom = size_t(32) << 20;
 constexpr int kMaxThreads = 6;
 // how long a thread looks for the next chunk (or the caller for a free buffer)
-// before it sleeps: chunks land every 10 us, waking takes several times that
-constexpr std::chrono::microseconds kLook{50};
+// before it sleeps: chunks land every 10 us, waking takes several times that, and
+// the copies of a served chunk follow one another in 100 us (six cavities of 20..60
+// with their fields 2.01 ms with 50 us, 1.71 with 300; thirty of 24..96 50.9 and 49.0)
+constexpr std::chrono::microseconds kLook{300};
 
 // One copy at a time (Shared::in_use).  Chunk i passes through buffer i % kRing:
 // the caller issues its transfer once chunk i - kRing has left the buffer,
@@ -62,8 +65,11 @@ public:
   {
     std::unique_ptr<Pool> p(new (std::nothrow) Pool);
     if (!p) return nullptr;
-    p->base_ = static_cast<char*>(std::aligned_alloc(kHugePage, kRing * kChunk));
-    if (!p->base_) return nullptr;
+    // mapped apart, so that the caller's heap stays as it is
+    void* const map = mmap(nullptr, kMapped, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (map == MAP_FAILED) return nullptr;
+    p->map_ = map;
+    p->base_ = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(map) + kHugePage - 1) / kHugePage * kHugePage);
     (void)madvise(p->base_, kRing * kChunk, MADV_HUGEPAGE);  // four pages to pin, not 2048
     std::memset(p->base_, 0, kRing * kChunk);
     p->pinned_ = cudaHostRegister(p->base_, kRing * kChunk, cudaHostRegisterPortable) == cudaSuccess;
@@ -90,7 +96,7 @@ public:
     for (std::thread& t : threads_) t.join();
     drop_events();
     if (pinned_) cudaHostUnregister(base_);
-    std::free(base_);
+    if (map_) munmap(map_, kMapped);
   }
 
   cudaError_t copy(char* dst, const char* src, size_t bytes, int device, cudaStream_t stream)
@@ -122,20 +128,30 @@ public:
     for (size_t& l : left_) l = 0;
     while (landed_ < chunks && e == cudaSuccess) {
       const size_t b = issued % kRing;
-      if (issued < chunks && issued < landed_ + kRing && left_[b] == issued / kRing) {
+      const bool issue = issued < chunks && issued < landed_ + kRing && left_[b] == issued / kRing;
+      if (landed_ < issued) {
+        // handed out as soon as it is there, also between two transfers' issues
+        const cudaEvent_t ev = events_[landed_ % kRing];
+        lock.unlock();
+        const cudaError_t there = issue ? cudaEventQuery(ev) : cudaEventSynchronize(ev);
+        if (there == cudaErrorNotReady) (void)cudaGetLastError();
+        lock.lock();
+        if (there == cudaSuccess) {
+          if (++landed_ == 1) wake_.notify_all();
+          else wake_.notify_one();
+          continue;
+        }
+        if (there != cudaErrorNotReady) {
+          e = there;
+          continue;
+        }
+      }
+      if (issue) {
         const size_t at = issued++ * kChunk;
         lock.unlock();
         e = cudaMemcpyAsync(base_ + b * kChunk, src + at, std::min(kChunk, bytes - at), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaEventRecord(events_[b], stream);
         lock.lock();
-      } else if (landed_ < issued) {
-        lock.unlock();
-        e = cudaEventSynchronize(events_[landed_ % kRing]);
-        lock.lock();
-        if (e == cudaSuccess) {
-          if (++landed_ == 1) wake_.notify_all();
-          else wake_.notify_one();
-        }
       } else if (!write_one(lock)) {
         const size_t seen = written_;
         wait(lock, freed_, [&] { return written_ != seen; });
@@ -200,7 +216,8 @@ private:
     }
   }
 
-  char* base_ = nullptr;
+  void* map_ = nullptr;
+  char* base_ = nullptr;  // in map_, on a huge page
   bool pinned_ = false;
   std::vector<std::thread> threads_;
   std::mutex mutex_;
